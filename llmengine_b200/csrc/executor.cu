@@ -50,6 +50,8 @@ typedef int (*LatentPostFn)(const LlmeLatentPostArgs*, int, cudaStream_t);
 typedef int (*LatentAttnPlainFn)(const LlmeLatentAttnArgs*, int, cudaStream_t);
 typedef int (*LatentAttnTcFn)(const LlmeFastAttnArgs*, const float*, int, int, cudaStream_t);
 typedef int (*LatentFitsFn)(int);
+typedef int (*LatentPairFn)(const LlmeFastAttnArgs*, long long, long long, const float*, int, int, cudaStream_t);
+typedef int (*LatentPairFitsFn)(int, int);
 typedef int (*PostNormFn)(float*, const void*, int, const void*, int, void*, int, int, int, float, int, cudaStream_t);
 typedef int (*GatedActFn)(const void*, long long, void*, long long, int, int, int, int, float, float, cudaStream_t);
 typedef int (*GemmGatedFn)(const void*, long long, const void*, long long, void*, int, long long, int, int, int, int, float, float, cudaStream_t);
@@ -675,7 +677,13 @@ int op_latent_attention(LlmeExecutor& ex, const LlmeLatentAttentionOp& o, const 
         f.page_size = g.page_size; f.scale = o.scale; f.window = o.window;
         if (s.num_portion > 0) {
             f.rows = s.portion_rows; f.n_rows = s.num_portion; f.splits = 1;
-            if (int rc = ex.launched(tc(&f, o.sink, o.rot, s.max_portion_len, st), "latent_attention_tc")) return rc;
+            // On tcgen05 where the latent size and the pages allow it: 128 keys of 128 (token, head) rows take a pair of blocks 3.2 us there, 32
+            // keys of 64 rows 4.3 us of the warp-level kernel's block, so it is ahead from the shortest portion on.
+            auto* pair = (LatentPairFn)ex.find_hd("latent_pair", o.rank);
+            auto* pair_fits = (LatentPairFitsFn)ex.find_hd("latent_pair_supports", o.rank);
+            if (pair && pair_fits && ex.choice("attention.portion") == "tcgen05" && pair_fits(o.rot, g.page_size) && aligned16(o.q, o.cache, o.out)) {
+                if (int rc = ex.launched(pair(&f, (long long)s.num_tokens * o.nh, o.cache_rows, o.sink, o.rot, s.max_portion_len, st), "latent_pair")) return rc;
+            } else if (int rc = ex.launched(tc(&f, o.sink, o.rot, s.max_portion_len, st), "latent_attention_tc")) return rc;
         }
         if (s.num_decode > 0) {
             f.rows = s.decode_rows; f.n_rows = s.num_decode;

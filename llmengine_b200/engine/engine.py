@@ -433,5 +433,7 @@ class Engine:
         for key in libs:
             if key.startswith("attention_tc@HEAD_DIM="):
                 status = status or int(libs[key].llme_attention_tc_status())
+            if key.startswith("attention_latent_tcgen05@"):
+                status = status or int(libs[key].llme_latent_pair_status())
         if status:
             raise RuntimeError(f"a tcgen05 kernel gave up waiting (code {status}): its results are not valid")

@@ -32,6 +32,8 @@ SOURCES: Dict[str, str] = {
     "attention_latent": "attention_latent.cu",
     # the same on the tensor cores, per latent size (a multiple of 64): "attention_latent_tc@RANK=512"
     "attention_latent_tc": "attention_latent_tc.cu",
+    # its prompt portions on tcgen05, per latent size (a multiple of 128 up to 512): "attention_latent_tcgen05@RANK=512"
+    "attention_latent_tcgen05": "attention_latent_tcgen05.cu",
     # attention with keys and values of different widths, a window that keeps the first positions, and a sink
     "attention_window": "attention_window.cu",
     # the same on the tensor cores, per pair of sizes: "attention_window_tc@DK=64,DV=64"
@@ -77,6 +79,7 @@ VARIANTS: Dict[str, List[str]] = {
     "attention_tc": ["attention_tc@HEAD_DIM=64", "attention_tc@HEAD_DIM=128", "attention_tc@HEAD_DIM=64,VALUE_DIM=128,MAPS=2"],
     "attention_maps": ["attention_maps@DK=64,DV=128"],
     "attention_latent_tc": ["attention_latent_tc@RANK=128", "attention_latent_tc@RANK=512"],
+    "attention_latent_tcgen05": ["attention_latent_tcgen05@RANK=128", "attention_latent_tcgen05@RANK=512"],
     "attention_window_tc": ["attention_window_tc@DK=64,DV=64", "attention_window_tc@DK=128,DV=128"],
 }
 

@@ -215,6 +215,7 @@ class CudaOps:
         "attention_latent": {"latent_attention_plain": "llme_latent_attention_plain"},
         "attention_latent_tc": {"latent_attention_tc/{hd}": "llme_latent_attention_tc",
                                 "latent_attention_tc_fits/{hd}": "llme_latent_attention_tc_fits"},
+        "attention_latent_tcgen05": {"latent_pair/{hd}": "llme_latent_pair", "latent_pair_supports/{hd}": "llme_latent_pair_supports"},
         "gemm_skinny": {"gemm_skinny": "llme_gemm_skinny_bf16", "gemm_skinny_swiglu": "llme_gemm_skinny_swiglu_bf16",
                         "gemm_skinny_act": "llme_gemm_skinny_act_bf16", "gemm_skinny_gated": "llme_gemm_skinny_gated_bf16"},
         "gemm_tcgen05": {"gemm_tc": "llme_gemm_tc_bf16", "gemm_tc_swiglu": "llme_gemm_tc_swiglu_bf16",
@@ -288,6 +289,8 @@ class CudaOps:
                 want("attention_latent")
                 if fast_attention and self.latent_tc_supports(a["kv_rank"], a["rot_dim"], a["q"].dtype):
                     want(f"attention_latent_tc@RANK={a['kv_rank']}")
+                    if a["kv_rank"] % 128 == 0 and a["kv_rank"] <= 512 and self.chosen("attention.portion") == "tcgen05":
+                        want(f"attention_latent_tcgen05@RANK={a['kv_rank']}")
             if op.kind == "batched_linear" and a["x"].dtype == torch.float32:
                 want("gemm_f32")
             if op.kind == "token_side":
