@@ -115,6 +115,9 @@ struct TcAttnArgs {
     int max_blocks, n_rows, nh, nkv, page_size, window;
     float scale;
     float diff_weight, diff_scale, diff_eps;     // two maps: what a row's two outputs become (out is then [T, nh / 2, VD])
+    const float* sink;           // [nh] or null: a logit that only joins the denominator
+    int keep_first;              // beside a window: the first positions of the request are always seen
+    float softcap;               // c > 0: a score s becomes c tanh(s / c) behind the scale
 };
 #include "kernel_args.h"
 static_assert(sizeof(TcAttnArgs) == sizeof(LlmeTcAttnArgs), "the argument block must match kernel_args.h");
@@ -283,6 +286,9 @@ struct Barriers {
     float row_max[QT][2][2][BM];  // [Q tile][tile parity][half][row]: the halves' maxima of a key tile
 };
 
+// EXT: with a sink, kept first positions or a cap on the scores (a form of its own, so that plain attention does not carry them).  Two
+// prompts of 1,900 tokens in all, 16 / 4 heads of 128, a window of 1,024 and four kept positions take 47 us, 134 us on the warp-level kernel.
+template <bool EXT>
 __global__ void __launch_bounds__(THREADS, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                     TcAttnArgs a) {
@@ -313,8 +319,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int t_lo = m0 / G, t_hi = min(q_len - 1, (m0 + row_tiles * BM - 1) / G);
     const int hi_max = start + t_hi;                                  // last key any row of the block sees
     const int lo_min = a.window > 0 ? max(0, start + t_lo - a.window + 1) : 0;
+    const int ctx = start + q_len;
     const int tile_first = lo_min / BN, tile_last = hi_max / BN;
-    const int n_tiles = tile_last - tile_first + 1;
+    // in front of the window's tiles, those of the kept first positions that they do not hold
+    const int n_first = EXT && a.window > 0 ? min((a.keep_first + BN - 1) / BN, tile_first) : 0;
+    const int n_tiles = n_first + tile_last - tile_first + 1;
+    auto tile_no = [&](int i) { return EXT && i < n_first ? i : tile_first - n_first + i; };
 
     if (threadIdx.x == 0) {
         mbar_init(&bar->q_full, 1);
@@ -376,8 +386,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         struct BoxRows { long long k, v; };                               // rows of this lane's box in the key and in the value map, or -1
         bool ok = true;
         auto first_row = [&](int i) -> BoxRows {
-            const int ja = (tile_first + i) * BN + (my_box << box_shift);
-            if (i >= n_tiles || my_box >= n_boxes || ja + rows_per_box - 1 < lo_min || ja > hi_max) return {-1, -1};
+            const int ja = tile_no(i) * BN + (my_box << box_shift);
+            if (i >= n_tiles || my_box >= n_boxes || (ja + rows_per_box - 1 < lo_min && !(EXT && ja < a.keep_first)) || ja > hi_max) return {-1, -1};
             const int blk = ps_shift >= 0 ? ja >> ps_shift : ja / ps;
             const long long page = bt[blk], off = ja - blk * ps;
             return {page * key_page + key_head + off, page * value_page + value_head + off};
@@ -385,9 +395,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // One load of a tile: its keys (which = 0) or its values (1), into the stage i % 2; `full` counts its bytes,
         // `empty` (if any) with `empty_parity` says when the stage may be overwritten.
         auto load_tile = [&](int i, int which, long long my_row, unsigned long long* full, unsigned long long* empty, unsigned empty_parity) {
-            const int j0 = (tile_first + i) * BN;
+            const int j0 = tile_no(i) * BN;
             const int ja = j0 + (my_box << box_shift), jb = ja + rows_per_box - 1;
-            const bool whole = my_row >= 0 && ja >= lo_min && jb <= hi_max;
+            // (a page that is held is finite up to the request's last token, whatever the block sees of it: scores of keys that a row
+            // does not see are masked)
+            const bool whole = my_row >= 0 && jb < ctx;
             const unsigned whole_mask = __ballot_sync(0xffffffffu, whole);                 // one bit per TMA load
             const unsigned part_mask = __ballot_sync(0xffffffffu, my_row >= 0 && !whole && my_half == 0);
             const unsigned tx = (unsigned)__popc(whole_mask) * load_bytes;
@@ -395,8 +407,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (empty) ok = mbar_wait(empty, empty_parity, abort_flag, 10 + which);
             ok = ok && !*abort_flag;
             if (!ok) return;
-            // First the boxes that straddle an edge of the visible range: they are copied by hand, visible
-            // rows only, the rest zeroed.  Then, after those writes are published, one lane arms the barrier
+            // First the box that the request ends in: it is copied by hand, the rows behind the last token
+            // zeroed.  Then, after those writes are published, one lane arms the barrier
             // and the lanes start the TMA loads of the boxes that are needed whole.
             if (part_mask) {
                 for (unsigned rest = part_mask; rest; rest &= rest - 1) {
@@ -407,7 +419,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         const int j = j0 + b + rr;
                         const int h = ch >> 3, q = ch & 7, row = b + rr;
                         uint4 v = make_uint4(0, 0, 0, 0);
-                        if (j >= lo_min && j <= hi_max)
+                        if (j < ctx)
                             v = *reinterpret_cast<const uint4*>(MAPS == 2 && !which ? a.cache + (row0 + (long long)h * ps + rr) * HD + q * 8
                                                                                     : a.cache + (row0 + rr) * VD + ch * 8);
                         *reinterpret_cast<uint4*>(tile + h * HALF_BYTES + row * 128 + ((q ^ (row & 7)) << 4)) = v;
@@ -545,8 +557,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const int p = start + min(m, M - 1) / G;         // its position
             const int phi = row_ok ? p : -1;
             const int plo = a.window > 0 ? max(0, p - a.window + 1) : 0;
+            const int kept = EXT ? a.keep_first : 0;
             const unsigned lane_off = (unsigned)(quarter * 32) << 16;
-            const float sc = a.scale * LOG2E;
+            const bool capped = EXT && a.softcap > 0.0f;
+            const float to_cap = capped ? a.scale / a.softcap : 0.0f;
+            const float sc = capped ? a.softcap * LOG2E : a.scale * LOG2E;       // (behind the cap a score is tanh(.))
             // what every row of this warp sees entirely, without a mask
             const int warp_p_lo = start + min(q_len - 1, (mt0 + quarter * 32) / G);
             const int warp_p_hi = start + min(q_len - 1, (mt0 + quarter * 32 + 31) / G);
@@ -554,10 +569,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const bool warp_full = mt0 + quarter * 32 + 31 < M;
             // the two warps of a (Q tile, quarter) meet at a named barrier of their own (64 threads)
             auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + t * 4 + quarter) : "memory"); };
-            float m_ref = -INFINITY, l_run = 0.0f;
+            const bool with_sink = EXT && a.sink && row_ok;
+            float m_ref = with_sink ? a.sink[kvh * G + m % G] * LOG2E : -INFINITY;
+            float l_run = with_sink && ch == 0 ? 1.0f : 0.0f;              // the sink counts once
             bool ok = true;
             for (int i = 0; i < n_tiles; ++i) {
-                const int j0 = (tile_first + i) * BN;
+                const int j0 = tile_no(i) * BN;
                 unsigned pk[32];
                 const int s2 = i & 1;
                 ok = ok && mbar_wait(&bar->s_full[t], i & 1, abort_flag, 30);
@@ -575,11 +592,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     for (int c0 = 0; c0 < BH; c0 += 32) {
                         float v[32];
                         tmem_ld32(tmem_s[t] + lane_off + (unsigned)(ch * BH + c0), v);
+                        if (EXT && capped) {
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) v[e] = tanhf(v[e] * to_cap);
+                        }
                         if (!unmasked) {
 #pragma unroll
                             for (int e = 0; e < 32; ++e) {
                                 const int j = j0 + ch * BH + c0 + e;
-                                if (j < plo || j > phi) v[e] = -INFINITY;
+                                if ((j < plo && !(EXT && j < kept)) || j > phi) v[e] = -INFINITY;
                             }
                         }
                         if (with_max) {
@@ -634,7 +655,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                                 tmem_st32(tmem_o[t] + lane_off + (unsigned)(ch * OC + c), v);
                             }
                         } else if (move) {
-                            l_run *= fast_exp2(m_ref - ref);         // first tile: nothing accumulated yet (and l_run is 0)
+                            l_run *= fast_exp2(m_ref - ref);         // first tile: nothing accumulated yet (l_run is 0, or the sink's)
                         }
                         m_ref = m_new;
                         if (ok) half_pass(ref, false);
@@ -834,16 +855,19 @@ LLME_API int llme_attention_tc(const void* q, long long q_tokens, long long tota
     CUresult r = cache_map(&mk, HD, total_cache_rows);
     if (r == CUDA_SUCCESS) r = cache_map(&mv, VD, total_cache_rows / MAPS);
     if (r != CUDA_SUCCESS) LLME_REFUSE("attention_tc: cuTensorMapEncodeTiled (cache) failed with code %d", (int)r);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    const bool ext = a.sink || (a.keep_first > 0 && a.window > 0) || a.softcap > 0.0f;
+    if (ext && MAPS == 2) LLME_REFUSE("attention_tc: the form for two maps takes no sink, kept first positions or cap");
+    auto kernel = ext ? attention_tc_kernel<MAPS == 1> : attention_tc_kernel<false>;
+    static bool configured[2] = {false, false};
+    if (!configured[ext]) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
         if (e != cudaSuccess) LLME_REFUSE("attention_tc: cannot reserve %zu bytes of shared memory: %s", SMEM_BYTES, cudaGetErrorString(e));
-        configured = true;
+        configured[ext] = true;
     }
     const long long tiles = ((long long)max_q_len * G + BLOCK_ROWS - 1) / BLOCK_ROWS;
     if (tiles * (a.nkv / MAPS) > 2147483647LL) LLME_REFUSE("attention_tc: grid too large");
     dim3 grid((unsigned)(tiles * (a.nkv / MAPS)), 1, a.n_rows);
-    attention_tc_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(mq, mk, mv, a);
+    kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(mq, mk, mv, a);
     LLME_LAUNCH_STATUS();
 }
 

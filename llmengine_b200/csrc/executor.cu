@@ -813,7 +813,16 @@ int window_attend(LlmeExecutor& ex, const LlmeWindowAttentionOp& o, const LlmeSt
         f.table_rows = s.state_slots; f.block_tables = g.block_tables; f.max_blocks = g.max_blocks; f.nh = o.nh; f.nkv = o.nkv;
         f.page_size = g.page_size; f.window = o.window; f.keep_first = o.keep_first; f.scale = o.scale; f.softcap = o.softcap;
         f.value_share = o.value_share;
-        if (s.num_portion > 0) {
+        // prompt portions over keys and values of one width: the tcgen05 kernel with a sink, kept first positions and a cap (47 us against
+        // 134 us of the warp-level kernel for 1,900 tokens of 16 / 4 heads of 128)
+        const int rep = o.nh / o.nkv, ps = g.page_size;
+        auto* big = o.dk == o.dv && o.value_share <= 1 ? (AttnTcFn)ex.find_hd("attention_tc", o.dk) : nullptr;
+        if (s.num_portion > 0 && big && ex.choice("attention.portion") == "tcgen05" && ps >= 8 && (ps <= 128 ? 128 % ps == 0 : ps % 128 == 0) && 128 % rep == 0 &&
+            aligned16(o.q, o.cache, o.out)) {
+            LlmeTcAttnArgs a = {o.out, o.cache, s.portion_rows, s.cu_q_lens, s.ctx_lens, s.state_slots, g.block_tables, g.max_blocks, s.num_portion, o.nh,
+                                o.nkv, ps, o.window, o.scale, 0.0f, 0.0f, 0.0f, o.sink, o.keep_first, o.softcap};
+            if (int rc = ex.launched(big(o.q, s.num_tokens, o.cache_pages * 2 * o.nkv * ps, &a, s.max_portion_len, st), "attention_tc")) return rc;
+        } else if (s.num_portion > 0) {
             f.rows = s.portion_rows; f.n_rows = s.num_portion;
             if (int rc = ex.launched(tc(&f, s.max_portion_len, 0, st), "window_attention_tc")) return rc;
         }

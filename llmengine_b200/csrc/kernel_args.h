@@ -46,6 +46,8 @@ typedef struct LlmeTcAttnArgs {
     int max_blocks, n_rows, nh, nkv, page_size, window;
     float scale;
     float diff_weight, diff_scale, diff_eps;     /* the form for two maps: out = (a1 - weight a2) / rms * scale, [T, nh / 2, dv] */
+    /* all off when zero: a learned logit per head that joins the denominator; first positions seen beside a window; s -> c tanh(s / c) */
+    const float* sink; int keep_first; float softcap;
 } LlmeTcAttnArgs;
 
 /* Norm of the latent, rotation of the shared key part and of the heads' rotated query parts, cache write. */

@@ -92,6 +92,7 @@ class _TcAttnArgs(Structure):
         ("table_rows", c_void_p), ("block_tables", c_void_p),
         ("max_blocks", c_int), ("n_rows", c_int), ("nh", c_int), ("nkv", c_int), ("page_size", c_int),
         ("window", c_int), ("scale", c_float), ("diff_weight", c_float), ("diff_scale", c_float), ("diff_eps", c_float),
+        ("sink", c_void_p), ("keep_first", c_int), ("softcap", c_float),
     ]
 
 
@@ -277,6 +278,8 @@ class CudaOps:
                         want(f"attention_tc@HEAD_DIM={a['qk_dim']}")
                 elif fast_attention and build.has_source("attention_window_tc") and self.window_tc_supports(a["qk_dim"], a["v_dim"], a["q"].dtype):
                     want(f"attention_window_tc@DK={a['qk_dim']},DV={a['v_dim']}")
+                    if a["qk_dim"] == a["v_dim"] and a["qk_dim"] in (64, 128) and a.get("value_share", 1) <= 1 and self.chosen("attention.portion") == "tcgen05":
+                        want(f"attention_tc@HEAD_DIM={a['qk_dim']}")
             if op.kind in ("moe_route", "grouped_linear", "moe_combine"):
                 want("moe")
             if op.kind == "grouped_linear" and a["x"].dtype == torch.bfloat16 and self.chosen("linear") != "plain" and build.has_source("moe_tc"):
