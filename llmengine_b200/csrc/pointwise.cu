@@ -328,6 +328,109 @@ __global__ void latent_post_kernel(LlmeLatentPostArgs a) {
     }
 }
 
+// The same for bfloat16 rows in 16-byte pieces: the block forms its token's cosines and sines once, and a thread finishes eight
+// coordinates at a time (with their partners, another piece or, for neighbouring pairs, the same one).  The form above forms a sine
+// and a cosine per coordinate and goes value by value: 21 us for 2,000 tokens of 16 heads with 512 + 64, 8.8 us here (caches cold).
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(p);
+    const unsigned w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+        v[2 * i] = f.x;
+        v[2 * i + 1] = f.y;
+    }
+}
+__device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&v)[8]) {
+    unsigned w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        w[i] = *reinterpret_cast<const unsigned*>(&h);
+    }
+    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+template <typename G>
+__global__ void __launch_bounds__(128) latent_post_pieces_kernel(LlmeLatentPostArgs a) {
+    extern __shared__ float turn[];                     // [rot_dims / 2] cosines, then sines
+    __shared__ float scratch[32];
+    typedef __nv_bfloat16 bf;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = blockIdx.x, rank = a.rank, rot = a.rot, width = rank + rot, half = rot > 0 ? a.rot_dims >> 1 : 0;
+    const int pos = a.positions[t];
+    for (int i = threadIdx.x; i < half; i += blockDim.x) {
+        float s, c;
+        sincosf((float)pos * a.inv_freq[i], &s, &c);
+        turn[i] = c * a.amplitude;
+        turn[half + i] = s * a.amplitude;
+    }
+    __syncthreads();
+    // coordinates j .. j + 7 of a vector of `rot`
+    auto rotate8 = [&](const bf* v, int j, bf* out) {
+        float x[8];
+        load8(v + j, x);
+        if (j < 2 * half && a.interleaved) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                const float c = turn[(j + e) >> 1], s = turn[half + ((j + e) >> 1)], u = x[e], w = x[e + 1];
+                x[e] = u * c - w * s;
+                x[e + 1] = w * c + u * s;
+            }
+        } else if (j < 2 * half) {
+            const bool first = j < half;
+            const int i = first ? j : j - half;
+            float o[8];
+            load8(v + (first ? j + half : j - half), o);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float c = turn[i + e], s = turn[half + i + e];
+                x[e] = first ? x[e] * c - o[e] * s : x[e] * c + o[e] * s;
+            }
+        }
+        store8(out + j, x);
+    };
+    const bf* kv = (const bf*)a.kv_in + (size_t)t * a.kv_stride;
+    const int slot = a.slot_mapping ? a.slot_mapping[t] : -1;
+    bf* row = (a.cache && slot >= 0) ? (bf*)a.cache + (size_t)slot * width : nullptr;
+    if (row) {                                          // uniform over the block
+        float ss = 0.0f;
+        for (int j = 8 * threadIdx.x; j < rank; j += 8 * blockDim.x) {
+            float v[8];
+            load8(kv + j, v);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) ss += v[e] * v[e];
+        }
+        ss = block_sum(ss, scratch);
+        const float rinv = 1.0f / sqrtf(ss / (float)rank + a.eps);
+        const G* gain = (const G*)a.c_gain;
+        for (int j = 8 * threadIdx.x; j < rank; j += 8 * blockDim.x) {
+            float v[8];
+            load8(kv + j, v);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = (v[e] * rinv) * to_f32(gain[j + e]);
+            store8(row + j, v);
+        }
+        for (int j = 8 * threadIdx.x; j < rot; j += 8 * blockDim.x) rotate8(kv + rank, j, row + rank);
+    }
+    if (rot > 0 && a.q_rot && a.q) {
+        const bf* qr = (const bf*)a.q_rot + (size_t)t * a.q_rot_stride;
+        bf* q = (bf*)a.q + (size_t)t * a.nh * width;
+        const int pieces = rot >> 3;
+        for (int e = threadIdx.x; e < a.nh * pieces; e += blockDim.x) {
+            const int h = e / pieces, j = 8 * (e - h * pieces);
+            rotate8(qr + (size_t)h * a.q_rot_head_stride, j, q + (size_t)h * width + rank);
+        }
+    }
+}
+
+static bool latent_pieces(const LlmeLatentPostArgs& a, int dtype) {
+    if (dtype != LLME_BF16 || a.rank % 8 || a.rot % 8 || a.rot > 4096 || (a.rot > 0 && a.rot_dims % (a.interleaved ? 8 : 16))) return false;
+    if (a.kv_stride % 8 || (a.q_rot && (a.q_rot_stride % 8 || a.q_rot_head_stride % 8))) return false;
+    return ((uintptr_t)a.kv_in | (uintptr_t)a.q_rot | (uintptr_t)a.q | (uintptr_t)a.cache) % 16 == 0;
+}
+
 LLME_API int llme_latent_post(const LlmeLatentPostArgs* args, int dtype, cudaStream_t stream) {
     const LlmeLatentPostArgs& a = *args;
     if (a.tokens <= 0) return 0;
@@ -336,10 +439,19 @@ LLME_API int llme_latent_post(const LlmeLatentPostArgs* args, int dtype, cudaStr
     if (a.rot > 0 && (!a.inv_freq || a.rot_dims <= 0 || a.rot_dims % 2 || a.rot_dims > a.rot))
         LLME_REFUSE("latent_post: %d rotated coordinates of %d need frequencies and an even count", a.rot_dims, a.rot);
     const int threads = 128;
+    // (up to 256 tokens the blocks below, of which a token has several, are through before a table is formed: 24 tokens of 16 heads
+    // take a layer 90.3 us so, 92.1 us in pieces)
+    if (a.tokens > 256 && latent_pieces(a, dtype) && (a.gain_dtype == LLME_BF16 || a.gain_dtype == LLME_F32)) {
+        const dim3 pieces_grid(a.tokens);
+        const size_t smem = (size_t)(a.rot > 0 ? a.rot_dims : 0) * sizeof(float);
+        if (a.gain_dtype == LLME_F32) llme_launch(latent_post_pieces_kernel<float>, pieces_grid, dim3(threads), smem, stream, a);
+        else llme_launch(latent_post_pieces_kernel<__nv_bfloat16>, pieces_grid, dim3(threads), smem, stream, a);
+        LLME_LAUNCH_STATUS();
+    }
     // block (t, 0) norms, rotates and stores the token's cache row; blocks (t, 1..) rotate the heads' query parts
     int q_blocks = a.rot > 0 && a.q_rot ? (a.nh * a.rot + threads - 1) / threads : 0;
     if (q_blocks > 8) q_blocks = 8;
-    if (a.tokens > 256) q_blocks = q_blocks ? 1 : 0;
+    if (a.tokens > 256) q_blocks = q_blocks ? 1 : 0;      // (what does not come in pieces)
     const dim3 grid(a.tokens, 1 + q_blocks);
 #define LLME_LP(T, G) llme_launch(latent_post_kernel<T, G>, grid, dim3(threads), 0, stream, a)
     if (dtype == LLME_F32 && a.gain_dtype == LLME_F32) LLME_LP(float, float);
