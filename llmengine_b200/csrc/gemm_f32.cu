@@ -1,8 +1,20 @@
 // True 32-bit matrix product C[M,N] = A[M,K] * W[N,K]^T on the CUDA cores (FMA, no
-// tensor cores, no reduced-precision mode).  Every output element is one accumulator
-// that adds its K products in the order k = 0..K-1, so a row's result does not depend
-// on how many other rows are in the launch.  It is the matrix product of the whole
+// tensor cores, no reduced-precision mode).  It is the matrix product of the whole
 // 32-bit path and the plain twin that the tensor-core kernels are checked against.
+//
+// K is cut into S segments of equal length, S = K / 1024 between 1 and 8; every output element adds the products of a
+// segment in the order of k, and then the segments' sums in their order.  S depends on K alone, so a row's result does not
+// depend on how many other rows are in the launch, whichever of the forms below serves it:
+//
+//   * a block walks all segments of its tile and adds each to C;
+//   * a cluster of S blocks, one segment each: the blocks leave their sums in shared memory, and each adds a share of the tile
+//     over the blocks in their order.  It fills the GPU where the tiles alone do not (300 x 2048 has 80 tiles of 64 x 128).
+//
+// 16 x 16 threads hold TM x TN outputs each, as packed pairs of neighbouring columns (fma.rn.f32x2: one instruction, each half
+// rounds as fmaf does); operands lie in shared memory k by k, two stages, the next one on its way through registers.
+// Bound by the multiply-adds: 300 x 11008 x 2048 takes 376 us and 300 x 2048 x 5504 216 us (36 and 31 TFLOP/s of 74; 2,048 rows: 50
+// and 44); one block per 64 x 64 tile with 4 x 4 outputs a thread, whatever the shape, took 675 and 617 us.  One row: 117 and 66 us
+// against 275 and 616 us.
 //
 // Reference counterparts: sgemm_nt_kernel (src/runtime/kernels/cuda_kernels.cu:282-294,
 // one thread per output, no tiling) and the cublasSgemm call of sgemm_nt_cublas (:892-908).
@@ -10,63 +22,281 @@
 
 LLME_API const char* llme_last_error() { return llme_error_buffer(); }
 
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
+namespace {
+
+constexpr int BK = 16, THREADS = 256, MAX_SEGMENTS = 8;
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+// values k .. k + 3 of a row, zeros from `end` on
+template <typename T>
+__device__ __forceinline__ float4 row_piece(const T* row, int k, int end, bool vec) {
+    if (vec && k + 4 <= end) return load4(row + k);
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (k < end) v.x = to_f32(row[k]);
+    if (k + 1 < end) v.y = to_f32(row[k + 1]);
+    if (k + 2 < end) v.z = to_f32(row[k + 2]);
+    if (k + 3 < end) v.w = to_f32(row[k + 3]);
+    return v;
+}
 
 template <typename WT>
-__global__ void __launch_bounds__(256) gemm_nt_f32_kernel(const float* __restrict__ A, const WT* __restrict__ W,
-                                                          float* __restrict__ C, int M, int N, int K,
-                                                          long long lda, long long ldw, long long ldc,
-                                                          long long sa, long long sw, long long sc) {
-    A += (size_t)blockIdx.z * sa;          // one member of a batch of products per grid plane
-    W += (size_t)blockIdx.z * sw;
-    C += (size_t)blockIdx.z * sc;
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[BK][BN + 4];
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;          // 16 x 16 threads, each TM x TN outputs
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+struct Problem {
+    const float* A; const WT* W; float* C;
+    int M, N, K, segment, segments, vec_a, vec_w, vec_c;
+    long long lda, ldw, ldc, sa, sw, sc;
+};
 
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        // 64 x 16 elements per operand, 4 per thread; consecutive threads read consecutive k
+// The i-th of a thread's T rows (or columns) of a tile: four side by side, the next four 64 further on.
+template <int T> __device__ __forceinline__ int place(int t, int i) { return T == 1 ? t : (i / 4) * 64 + t * 4 + (i & 3); }
+
+template <int TM, int TN>
+struct Tile {
+    static constexpr int BM = 16 * TM, BN = 16 * TN;
+    float a[2][BK][BM + 4], w[2][BK][BN + 4];
+};
+
+template <typename WT, int TM, int TN, bool SPLIT>
+__global__ void __launch_bounds__(THREADS, 2) gemm_nt_f32_kernel(Problem<WT> g) {
+    constexpr int BM = 16 * TM, BN = 16 * TN, AL = (BM * BK / 4 + THREADS - 1) / THREADS, WL = BN * BK / 4 / THREADS;
+    static_assert(WL >= 1 && TN % 4 == 0, "a tile has at least 64 columns");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Tile<TM, TN>& sm = *reinterpret_cast<Tile<TM, TN>*>(smem_raw);
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int member = SPLIT ? (int)blockIdx.z / g.segments : (int)blockIdx.z, rank = SPLIT ? (int)blockIdx.z % g.segments : 0;
+    const float* A = g.A + (size_t)member * g.sa;          // one member of a batch of products
+    const WT* W = g.W + (size_t)member * g.sw;
+    float* C = g.C + (size_t)member * g.sc;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const bool vec_a = g.vec_a, vec_w = g.vec_w;
+
+    f32x2 acc[TM][TN / 2];
+    for (int seg = SPLIT ? rank : 0; seg < (SPLIT ? rank + 1 : g.segments); ++seg) {
+        const int k_begin = seg * g.segment, k_end = min(g.K, k_begin + g.segment);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int e = tid + i * 256;
-            const int r = e >> 4, kk = e & 15;
-            const int gm = m0 + r, gn = n0 + r, gk = k0 + kk;
-            As[kk][r] = (gm < M && gk < K) ? A[(size_t)gm * lda + gk] : 0.0f;
-            Ws[kk][r] = (gn < N && gk < K) ? to_f32(W[(size_t)gn * ldw + gk]) : 0.0f;
-        }
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
+        float4 pa[AL], pw[WL];
+        auto fetch = [&](int k0) {
+#pragma unroll
+            for (int i = 0; i < AL; ++i) {
+                const int e = tid + i * THREADS, r = e >> 2, k = k0 + (e & 3) * 4;
+                pa[i] = e < BM * BK / 4 && m0 + r < g.M ? row_piece(A + (size_t)(m0 + r) * g.lda, k, k_end, vec_a) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int i = 0; i < WL; ++i) {
+                const int e = tid + i * THREADS, r = e >> 2, k = k0 + (e & 3) * 4;
+                pw[i] = n0 + r < g.N ? row_piece(W + (size_t)(n0 + r) * g.ldw, k, k_end, vec_w) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+        };
+        auto put = [&](int s) {
+#pragma unroll
+            for (int i = 0; i < AL; ++i) {
+                const int e = tid + i * THREADS, r = e >> 2, k = (e & 3) * 4;
+                if (e < BM * BK / 4) {
+                    sm.a[s][k][r] = pa[i].x; sm.a[s][k + 1][r] = pa[i].y; sm.a[s][k + 2][r] = pa[i].z; sm.a[s][k + 3][r] = pa[i].w;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < WL; ++i) {
+                const int e = tid + i * THREADS, r = e >> 2, k = (e & 3) * 4;
+                sm.w[s][k][r] = pw[i].x; sm.w[s][k + 1][r] = pw[i].y; sm.w[s][k + 2][r] = pw[i].z; sm.w[s][k + 3][r] = pw[i].w;
+            }
+        };
+        fetch(k_begin);
+        put(0);
         __syncthreads();
+        int s = 0;
+        for (int k0 = k_begin; k0 < k_end; k0 += BK, s ^= 1) {
+            const bool more = k0 + BK < k_end;
+            if (more) fetch(k0 + BK);
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float a[TM], b[TN];
+            for (int kk = 0; kk < BK; ++kk) {
+                float a[TM];
+                f32x2 w[TN / 2];
+                if (TM == 1) a[0] = sm.a[s][kk][ty];
+                else
 #pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
+                    for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4*>(&a[i]) = *reinterpret_cast<const float4*>(&sm.a[s][kk][place<TM>(ty, i)]);
 #pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = Ws[kk][tx * TN + j];
+                for (int j = 0; j < TN; j += 4) {
+                    const ulonglong2 two = *reinterpret_cast<const ulonglong2*>(&sm.w[s][kk][place<TN>(tx, j)]);
+                    w[j / 2] = two.x;
+                    w[j / 2 + 1] = two.y;
+                }
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
+                for (int i = 0; i < TM; ++i) {
+                    const f32x2 aa = pack2(a[i], a[i]);
 #pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                    for (int j = 0; j < TN / 2; ++j) acc[i][j] = fma2(aa, w[j], acc[i][j]);
+                }
+            }
+            if (more) put(s ^ 1);
+            __syncthreads();
         }
-        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < (SPLIT ? 0 : TM); ++i) {
+            const int gm = m0 + place<TM>(ty, i);
+            if (gm >= g.M) continue;
+            float* row = C + (size_t)gm * g.ldc;
+#pragma unroll
+            for (int j = 0; j < TN; j += 4) {
+                const int gn = n0 + place<TN>(tx, j);
+                float v[4];
+                unpack2(acc[i][j / 2], v[0], v[1]);
+                unpack2(acc[i][j / 2 + 1], v[2], v[3]);
+                if (g.vec_c && gn + 4 <= g.N) {
+                    float4 o = make_float4(v[0], v[1], v[2], v[3]);
+                    if (seg > 0) {
+                        const float4 c = *reinterpret_cast<const float4*>(row + gn);
+                        o = make_float4(c.x + o.x, c.y + o.y, c.z + o.z, c.w + o.w);
+                    }
+                    *reinterpret_cast<float4*>(row + gn) = o;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (gn + e < g.N) row[gn + e] = seg > 0 ? row[gn + e] + v[e] : v[e];
+                }
+            }
+        }
     }
+    if (SPLIT) {
+        // this block's sums into its shared memory, then a share of the tile's rows over all blocks in their order
+        float* part = reinterpret_cast<float*>(smem_raw);  // [BM][BN] (the stages are done with)
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int gm = m0 + ty * TM + i;
-        if (gm >= M) continue;
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int gn = n0 + tx * TN + j;
-            if (gn < N) C[(size_t)gm * ldc + gn] = acc[i][j];
+            for (int j = 0; j < TN; j += 4) {
+                float4 o;
+                unpack2(acc[i][j / 2], o.x, o.y);
+                unpack2(acc[i][j / 2 + 1], o.z, o.w);
+                *reinterpret_cast<float4*>(part + place<TM>(ty, i) * BN + place<TN>(tx, j)) = o;
+            }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const unsigned mine = (unsigned)__cvta_generic_to_shared(part);
+        for (int e = rank * THREADS + tid; e < BM * BN / 4; e += g.segments * THREADS) {
+            float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (int from = 0; from < g.segments; ++from) {
+                unsigned at;
+                float4 v;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(mine + 16u * (unsigned)e), "r"(from));
+                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+                sum = from == 0 ? v : make_float4(sum.x + v.x, sum.y + v.y, sum.z + v.z, sum.w + v.w);
+            }
+            const int gm = m0 + e / (BN / 4), gn = n0 + (e % (BN / 4)) * 4;
+            if (gm >= g.M) continue;
+            float* row = C + (size_t)gm * g.ldc;
+            if (g.vec_c && gn + 4 <= g.N) *reinterpret_cast<float4*>(row + gn) = sum;
+            else {
+                if (gn < g.N) row[gn] = sum.x;
+                if (gn + 1 < g.N) row[gn + 1] = sum.y;
+                if (gn + 2 < g.N) row[gn + 2] = sum.z;
+                if (gn + 3 < g.N) row[gn + 3] = sum.w;
+            }
         }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");     // nobody leaves while its sums are read
     }
 }
+
+template <typename WT, int TM, int TN, bool SPLIT>
+int launch(const Problem<WT>& g, int batch, cudaStream_t stream) {
+    constexpr int BM = 16 * TM, BN = 16 * TN;
+    constexpr size_t stages = sizeof(Tile<TM, TN>), part = SPLIT ? (size_t)BM * BN * 4 : 0, smem = stages > part ? stages : part;
+    auto kernel = gemm_nt_f32_kernel<WT, TM, TN, SPLIT>;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) LLME_REFUSE("gemm_f32: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+        configured = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, SPLIT ? batch * g.segments : batch);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = (unsigned)g.segments;
+    cfg.attrs = attr;
+    cfg.numAttrs = SPLIT ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, g);
+    LLME_LAUNCH_STATUS();
+}
+
+int sm_count() {
+    static int n = [] {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) v = 148;
+        return v;
+    }();
+    return n;
+}
+
+// Which tile, and whether a cluster shares its segments: the least number of rounds times a block's work.  A block's rate relative to
+// that of 128 x 128 outputs: what its operands cost
+// beside the multiply-adds (two 16-byte loads from shared memory for 64 of them, one and a quarter for 8).
+template <typename WT>
+int dispatch(const Problem<WT>& g, int batch, cudaStream_t stream) {
+    const int bm[4] = {128, 64, 64, 16}, bn[4] = {128, 128, 64, 128};
+    const double rate[4] = {1.0, 0.9, 0.75, 0.3};
+    int best = -1;
+    double best_cost = 0.0;
+    for (int i = 0; i < 8; ++i) {
+        const int c = i >> 1, split = i & 1;
+        if (split && (g.segments == 1 || (long long)batch * g.segments > 65535)) continue;
+        if ((g.M + bm[c] - 1) / bm[c] > 65535) continue;
+        const long long tiles = (long long)((g.M + bm[c] - 1) / bm[c]) * ((g.N + bn[c] - 1) / bn[c]) * batch, blocks = split ? tiles * g.segments : tiles;
+        const double rounds = (double)((blocks + sm_count() - 1) / sm_count());
+        const double cost = rounds * bm[c] * bn[c] * (split ? g.segment + 64.0 : (double)g.K + 32.0 * g.segments) / rate[c];
+        if (best < 0 || cost < best_cost) { best = i; best_cost = cost; }
+    }
+    switch (best) {
+        case 0: return launch<WT, 8, 8, false>(g, batch, stream);
+        case 1: return launch<WT, 8, 8, true>(g, batch, stream);
+        case 2: return launch<WT, 4, 8, false>(g, batch, stream);
+        case 3: return launch<WT, 4, 8, true>(g, batch, stream);
+        case 4: return launch<WT, 4, 4, false>(g, batch, stream);
+        case 5: return launch<WT, 4, 4, true>(g, batch, stream);
+        case 6: return launch<WT, 1, 8, false>(g, batch, stream);
+        case 7: return launch<WT, 1, 8, true>(g, batch, stream);
+    }
+    LLME_REFUSE("gemm_f32: M = %d needs more than 65535 grid rows", g.M);
+}
+
+template <typename WT>
+int product(const float* A, const WT* W, float* C, int M, int N, int K, long long lda, long long ldw, long long ldc, int batch, long long sa,
+            long long sw, long long sc, cudaStream_t stream) {
+    Problem<WT> g = {A, W, C, M, N, K, 0, 0, 0, 0, 0, lda, ldw, ldc, sa, sw, sc};
+    g.segments = K / 1024 < 1 ? 1 : (K / 1024 > MAX_SEGMENTS ? MAX_SEGMENTS : K / 1024);
+    g.segment = ((K + g.segments - 1) / g.segments + BK - 1) / BK * BK;
+    g.segments = (K + g.segment - 1) / g.segment;
+    g.vec_a = (uintptr_t)A % 16 == 0 && lda % 4 == 0 && sa % 4 == 0;
+    g.vec_w = (uintptr_t)W % (4 * sizeof(WT)) == 0 && ldw % 4 == 0 && sw % 4 == 0;
+    g.vec_c = (uintptr_t)C % 16 == 0 && ldc % 4 == 0 && sc % 4 == 0;
+    return dispatch(g, batch, stream);
+}
+
+}  // namespace
 
 // A [M,K] row stride lda; W [N,K] row stride ldw (float or bfloat16); C [M,N] row stride ldc.
 // `batch` products in one launch: member b reads A + b * sa and W + b * sw and writes C + b * sc.
@@ -75,13 +305,13 @@ LLME_API int llme_gemm_nt_f32_batched(const float* A, const void* W, int w_dtype
                                       cudaStream_t stream) {
     if (M <= 0 || N <= 0 || batch <= 0) return 0;
     if (!A || !W || !C || K <= 0) LLME_REFUSE("gemm_f32: null pointer or non-positive K");
+    if (batch == 1) sa = sw = sc = 0;                      // (unused)
+    // (a batch whose rows lie between those of its other members has a row stride longer than the row)
     if (lda < K || ldw < K || ldc < N) LLME_REFUSE("gemm_f32: a row stride is shorter than the row");
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
-    if (grid.y > 65535 || batch > 65535) LLME_REFUSE("gemm_f32: M = %d or a batch of %d needs more than 65535 grid planes", M, batch);
-    if (w_dtype == LLME_F32) gemm_nt_f32_kernel<float><<<grid, 256, 0, stream>>>(A, (const float*)W, C, M, N, K, lda, ldw, ldc, sa, sw, sc);
-    else if (w_dtype == LLME_BF16) gemm_nt_f32_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(A, (const __nv_bfloat16*)W, C, M, N, K, lda, ldw, ldc, sa, sw, sc);
-    else LLME_REFUSE("gemm_f32: unsupported weight dtype %d", w_dtype);
-    LLME_LAUNCH_STATUS();
+    if ((M + 63) / 64 > 65535 || batch > 65535) LLME_REFUSE("gemm_f32: M = %d or a batch of %d needs more than 65535 grid planes", M, batch);
+    if (w_dtype == LLME_F32) return product(A, (const float*)W, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream);
+    if (w_dtype == LLME_BF16) return product(A, (const __nv_bfloat16*)W, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream);
+    LLME_REFUSE("gemm_f32: unsupported weight dtype %d", w_dtype);
 }
 
 LLME_API int llme_gemm_nt_f32(const float* A, const void* W, int w_dtype, float* C, int M, int N, int K,
