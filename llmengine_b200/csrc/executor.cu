@@ -223,19 +223,20 @@ const char* kind_name(int kind) {
 constexpr int SKINNY_ROWS = 16;      // most rows the weight-streaming product takes (gemm_skinny.cu)
 
 // Whether a product of M tokens goes to the weight-streaming kernel when the choice is "auto".  That kernel has one
-// block per group of 16 weight rows (8 gate + 8 up rows with the activation), two blocks resident per SM: it wins
-// against the library's product for up to 8 tokens when its blocks fill their waves (4096 rows: 256 blocks for 296
-// places, 5.5 TB/s on 4096 x 12288 against 3.1), and loses when a second wave is nearly empty (5120 rows: 320 blocks,
-// 4.5 TB/s on 5120 x 17408 against 5.6) or when 9 to 16 tokens double the operands it re-reads from L2 per block.
-// Where its waves of 296 are badly filled the kernel has a lighter form with three blocks per SM (444 places: 6.1 TB/s
-// on 5120 x 17408 / 25600, against 5.7 to 5.9 for the library); 7,168 rows (448 groups) fit neither and go to the library.
+// block per group of 16 weight rows (8 gate + 8 up rows with the activation), two blocks resident per SM.
+// Row groups that fit one round of places go there however few they are (measured at 1 / 8 / 16 tokens, this kernel against the
+// library: 2048 x 5504 takes 5.7 / 6.2 / 7.0 us against 14.4 / 14.2 / 9.6, 2048 x 2048 2.8 / 3.1 / 3.5 against 8.0 / 7.1 / 5.5,
+// 3072 x 2048 3.6 / 3.8 / 4.5 against 8.5 / 7.5 / 5.8, 4096 x 4096 6.9 / 7.3 / 8.4 against 14.6 / 12.5 / 10.0, 512 x 4096 3.2 / 3.6 / 4.2
+// against 7.7).
+// More of them: for up to 8 tokens when they fill their rounds (a second round that is nearly empty loses: 5120 rows, 320 blocks, 4.5
+// TB/s on 5120 x 17408 against 5.6), of 296 places or, in the kernel's lighter form with three blocks per SM, of 444 (6.1 TB/s on
+// 5120 x 17408 / 25600, against 5.7 to 5.9 for the library); 7,168 rows (448 groups) fit neither and go to the library.  9 to 16 tokens
+// double the operands that every group re-reads from L2, and there the library is ahead from the second round on
+// (6144 x 4096: 14.3 against 12.9 us; 24576 x 4096: 39.5 against 37.7).
 bool skinny_pays(const LlmeExecutor& ex, int M, long long row_groups) {
     const long long places = 2LL * ex.sms, waves = (row_groups + places - 1) / places;
-    // 9 to 16 tokens: only where the row groups are one well-filled round (4,096 rows: 256 groups).  There the kernel
-    // takes 8.0 / 20.0 us for 4096 x 4096 / 4096 x 12288 against 10.6 / 21.7 us; with more row groups, each re-reading
-    // the tokens' operands, the library is ahead (6144 x 4096: 14.3 against 12.9 us; 24576 x 4096: 39.5 against 37.7).
-    if (M > 8) return row_groups <= places && 10 * row_groups >= 8 * places;
-    if (4 * row_groups <= places) return true;          // a small product is bound by its launch, not by its waves
+    if (row_groups <= places) return true;
+    if (M > 8) return false;
     if (10 * row_groups >= 8 * waves * places) return true;
     // the kernel's lighter form, three blocks per SM: 444 places a round (gemm_skinny.cu chooses it by the same figures)
     const long long places3 = 3LL * ex.sms, waves3 = (row_groups + places3 - 1) / places3;

@@ -10,8 +10,8 @@
 // registers the instruction reads.  How many bytes are in flight is then a matter of registers and
 // resident warps, not of shared-memory stages.
 //
-// A block owns one group of 16 rows of W.  Its eight warps take the 64-wide chunks of K in turn (warp w:
-// chunks w, w+8, ...); at the end the eight partial sums of every output are added in a fixed order.  A
+// A block owns one group of 16 rows of W.  Its eight (or sixteen) warps take the 64-wide chunks of K in turn (warp w:
+// chunks w, w+8, ...); at the end their partial sums of every output are added in a fixed order.  A
 // token's result does not depend on how many other tokens are in the call.  (A grid of as many blocks as
 // the GPU keeps resident, each with an equal share of (row group, chunk) units and shared row groups
 // finished by the block that comes second, was measured and was slower: 14.7 against 12.4 us for
@@ -31,8 +31,6 @@ namespace {
 
 typedef __nv_bfloat16 bf16;
 constexpr int KC = 64;            // k values per chunk (two blocks of 32)
-constexpr int WARPS = 8;
-constexpr int THREADS = WARPS * 32;
 int g_dense = 0;                  // llme_gemm_skinny_dense()
 __device__ __forceinline__ void mma_bf16(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
                                          unsigned b0, unsigned b1) {
@@ -63,8 +61,11 @@ struct SkinnyArgs {
 // 2.1 to 3.6 TB/s against 4.1 to 5.2 TB/s).
 // UNROLL: chunks of K whose loads a warp issues together; BLOCKS: blocks that must fit an SM (2 with 4 chunks in flight,
 // 3 with 2: fewer bytes in flight per SM, but 444 places instead of 296 for the row groups of a product).
-template <int MT, typename O, int UNROLL, int BLOCKS>
-__global__ void __launch_bounds__(THREADS, BLOCKS) gemm_skinny_kernel(SkinnyArgs a) {
+// WARPS: 8, or 16 where there are no more row groups than SMs: a block then has an SM to itself, and its row group's bytes come
+// from twice as many warps (2048 x 5504, 8 / 16 tokens: 6.2 / 7.0 us, 7.4 / 8.9 us with 8 warps).
+template <int MT, typename O, int UNROLL, int BLOCKS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, BLOCKS) gemm_skinny_kernel(SkinnyArgs a) {
+    constexpr int THREADS = WARPS * 32;
     __shared__ float red[WARPS][MT * 8][16];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int quad = lane & 3, r = lane >> 2;
@@ -204,8 +205,10 @@ int launch(const SkinnyArgs& a, cudaStream_t s) {
     const long long w2 = (groups + p2 - 1) / p2 * p2, w3 = (groups + p3 - 1) / p3 * p3;          // places of the rounds taken
     const bool fills2 = 10LL * groups >= 8 * w2, fills3 = 10LL * groups >= 7 * w3;
     const bool dense = MT == 1 && (g_dense == 2 || (g_dense == 0 && !fills2 && fills3 && 4LL * groups > p2));
-    if (dense) llme_launch(gemm_skinny_kernel<MT, O, 2, 3>, dim3(groups), dim3(THREADS), 0, s, a);
-    else llme_launch(gemm_skinny_kernel<MT, O, 4, 2>, dim3(groups), dim3(THREADS), 0, s, a);
+    // (by the row groups alone: a token's result must not depend on how many others are in the call)
+    if (groups <= sm_count() && g_dense == 0) llme_launch(gemm_skinny_kernel<MT, O, 4, 1, 16>, dim3(groups), dim3(512), 0, s, a);
+    else if (dense) llme_launch(gemm_skinny_kernel<MT, O, 2, 3, 8>, dim3(groups), dim3(256), 0, s, a);
+    else llme_launch(gemm_skinny_kernel<MT, O, 4, 2, 8>, dim3(groups), dim3(256), 0, s, a);
     LLME_LAUNCH_STATUS();
 }
 
