@@ -4,10 +4,17 @@
 //
 // A block owns a tile of BM pairs of ONE expert x BN output columns and walks K in steps of 32 through a cp.async
 // pipeline of two or three stages; its four warps share the tile by columns (mma.sync m16n8k16, fragments by ldmatrix).
-// Two shapes: 64 x 64 where experts get many rows (prompts; tiles of 128 rows on eight warps were no faster, 406 against
-// 372 us for 2,048 tokens on 4 of 32 experts of 1,024: an expert's last tile is the emptier the larger the tiles are),
-// 16 x 128 where they get a few (decode steps: every weight tile is then read by exactly one block, which is all a
-// weight-streaming product can ask for).  The row tiles of all experts
+// Its shape is 64 x 64 (tiles of 128 rows on eight warps were no faster, 406 against
+// 372 us for 2,048 tokens on 4 of 32 experts of 1,024: an expert's last tile is the emptier the larger the tiles are).
+//
+// Where experts get a few rows (decode steps) the weights are streamed instead (grouped_skinny_kernel): a block owns 16 weight rows
+// of an expert (8 gate rows and the 8 up rows of the same outputs) as the M side of the instructions and up to 8 or 16 pairs as their
+// N side; its eight warps take 64 values of k in turn, every operand goes from memory straight into the registers that the
+// instruction reads (the order in which the products of a sum are added is free: four lanes take 8 consecutive values each), and
+// four chunks a warp are on their way at a time.  Tiles of 16 x 128 through shared memory, three steps of 32 values of k in flight a block,
+// took a mixture of 4 of 32 experts of 2,048 x 2,048 107 / 191 / 204 us at 2 / 8 / 24 tokens (the whole layer), this takes 54 / 110 / 164.
+//
+// The row tiles of all experts
 // are numbered one after the other and a block finds its expert from the offsets; a launch has as many row tiles as
 // any routing can need, and blocks beyond the step's own count leave at once.  A row's sums never depend on which
 // other rows share its tile.
@@ -39,19 +46,28 @@ __device__ __forceinline__ void mma_bf16(float* d, const unsigned* a, unsigned b
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ bool find_tile(const int* __restrict__ offsets, int E, int BM, int tile, int* expert, int* first, int* rows) {
+// Row tile `tile` of all experts' tiles of BM rows, looked for by a whole warp (32 experts at a time: one after the other their
+// offsets would be as many round trips to memory).
+__device__ __forceinline__ bool find_tile(const int* __restrict__ offsets, int E, int BM, int tile, int lane, int* expert, int* first, int* rows) {
     int seen = 0;
-    for (int e = 0; e < E; ++e) {
-        const int lo = offsets[e], n = offsets[e + 1] - lo;
-        const int tiles = (n + BM - 1) / BM;
-        if (tile < seen + tiles) {
-            const int at = (tile - seen) * BM;
-            *expert = e;
-            *first = lo + at;
-            *rows = n - at < BM ? n - at : BM;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+        const int e = e0 + lane, lo = offsets[e < E ? e : E], n = offsets[e < E ? e + 1 : E] - lo, tiles = (n + BM - 1) / BM;
+        int upto = tiles;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const int at = tile - (seen + upto - tiles);
+        const unsigned hit = __ballot_sync(0xffffffffu, at >= 0 && at < tiles);
+        if (hit) {
+            const int src = __ffs(hit) - 1, row = __shfl_sync(0xffffffffu, at, src) * BM, left = __shfl_sync(0xffffffffu, n, src) - row;
+            *expert = e0 + src;
+            *first = __shfl_sync(0xffffffffu, lo, src) + row;
+            *rows = left < BM ? left : BM;
             return true;
         }
-        seen += tiles;
+        seen += __shfl_sync(0xffffffffu, upto, 31);
     }
     return false;
 }
@@ -80,10 +96,10 @@ __global__ void __launch_bounds__(32 * WM * WNW) grouped_tc_kernel(LlmeGroupedAr
     __shared__ int s_src[BM], s_dst[BM];
     pdl_launch_dependents();
     pdl_wait();                                           // the offsets and the order come from the kernel before
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         int e = -1, first = 0, rows = 0;
-        if (!find_tile(a.offsets, a.num_experts, BM, blockIdx.y, &e, &first, &rows)) e = -1;
-        s_tile[0] = e; s_tile[1] = first; s_tile[2] = rows;
+        if (!find_tile(a.offsets, a.num_experts, BM, blockIdx.y, threadIdx.x, &e, &first, &rows)) e = -1;
+        if (threadIdx.x == 0) { s_tile[0] = e; s_tile[1] = first; s_tile[2] = rows; }
     }
     __syncthreads();
     const int e = s_tile[0], first = s_tile[1], rows = s_tile[2];
@@ -193,13 +209,121 @@ __global__ void __launch_bounds__(32 * WM * WNW) grouped_tc_kernel(LlmeGroupedAr
         }
 }
 
+// Few rows an expert.  MT: 8-pair tiles (a tile of 8 MT pairs of one expert).
+constexpr int KC = 64, SKINNY_WARPS = 8, UNROLL = 4;
+
+// weights are read by few blocks: do not keep them in L1
+__device__ __forceinline__ uint4 load_stream(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+template <int MT, int ACT, typename O>
+__global__ void __launch_bounds__(32 * SKINNY_WARPS, 2) grouped_skinny_kernel(LlmeGroupedArgs a) {
+    constexpr int BM = 8 * MT;
+    __shared__ float red[SKINNY_WARPS][BM][16];
+    __shared__ int s_tile[3], s_dst[BM];
+    pdl_launch_dependents();
+    pdl_wait();                                           // the offsets and the order come from the kernel before
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, r = lane >> 2;
+    if (warp == 0) {
+        int e = -1, first = 0, rows = 0;
+        if (!find_tile(a.offsets, a.num_experts, BM, blockIdx.y, lane, &e, &first, &rows)) e = -1;
+        if (lane == 0) { s_tile[0] = e; s_tile[1] = first; s_tile[2] = rows; }
+    }
+    __syncthreads();
+    const int e = s_tile[0], first = s_tile[1], rows = s_tile[2];
+    if (e < 0) return;
+    const int n_out = ACT == 1 ? a.n / 2 : a.n, rg = blockIdx.x;
+    // the pairs of this lane (pair lane / 4 of every tile of eight) and the weight rows (clamped: a row past the end is read, not stored)
+    const bf16* xr[MT];
+    bool xok[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+        xok[m] = m * 8 + r < rows;
+        const int at = first + (xok[m] ? m * 8 + r : 0), pair = a.order[at];
+        xr[m] = (const bf16*)a.x + (size_t)(a.gather ? pair / a.top_k : at) * a.ldx + quad * 8;
+        if (warp == 0 && quad == 0) s_dst[m * 8 + r] = a.scatter ? pair : at;
+    }
+    const int row0 = ACT == 1 ? min(rg * 8 + r, n_out - 1) : min(rg * 16 + r, n_out - 1);
+    const int row1 = ACT == 1 ? n_out + row0 : min(rg * 16 + r + 8, n_out - 1);
+    const bf16* w = (const bf16*)a.w + (size_t)e * a.w_expert;
+    const bf16* w0 = w + (size_t)row0 * a.ldw + quad * 8;
+    const bf16* w1 = w + (size_t)row1 * a.ldw + quad * 8;
+    float acc[MT][4];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.0f;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    const int chunks = (a.k + KC - 1) / KC;
+    for (int c = warp; c < chunks; c += UNROLL * SKINNY_WARPS) {
+        uint4 wa[UNROLL][2], wb[UNROLL][2], xv[UNROLL][MT][2];
+#pragma unroll
+        for (int q = 0; q < UNROLL; ++q)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const int k = (c + q * SKINNY_WARPS) * KC + b * 32;
+                const bool ok = k + quad * 8 < a.k;       // k is a multiple of 8: a piece is inside or outside
+                wa[q][b] = ok ? load_stream(w0 + k) : zero;
+                wb[q][b] = ok ? load_stream(w1 + k) : zero;
+#pragma unroll
+                for (int m = 0; m < MT; ++m) xv[q][m][b] = ok && xok[m] ? *reinterpret_cast<const uint4*>(xr[m] + k) : zero;
+            }
+#pragma unroll
+        for (int q = 0; q < UNROLL; ++q)
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const unsigned lo[4] = {wa[q][b].x, wb[q][b].x, wa[q][b].y, wb[q][b].y}, hi[4] = {wa[q][b].z, wb[q][b].z, wa[q][b].w, wb[q][b].w};
+                    mma_bf16(acc[m], lo, xv[q][m][b].x, xv[q][m][b].y);
+                    mma_bf16(acc[m], hi, xv[q][m][b].z, xv[q][m][b].w);
+                }
+    }
+    // the warps' partial sums, added in a fixed order
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) red[warp][m * 8 + quad * 2 + (i & 1)][r + (i >> 1) * 8] = acc[m][i];
+    __syncthreads();
+    auto total = [&](int tok, int row) {
+        float v = red[0][tok][row];
+#pragma unroll
+        for (int wp = 1; wp < SKINNY_WARPS; ++wp) v += red[wp][tok][row];
+        return v;
+    };
+    constexpr int COLS = ACT == 1 ? 8 : 16;
+    for (int i = threadIdx.x; i < BM * COLS; i += 32 * SKINNY_WARPS) {
+        const int tok = i / COLS, j = i % COLS, col = rg * COLS + j;
+        if (tok >= rows || col >= n_out) continue;
+        float v = total(tok, j);
+        if (ACT == 1)                                     // gate and up pass through bfloat16 first, as they do when the activation is a kernel of its own
+            v = silu_mul_bf16(__bfloat162float(__float2bfloat16_rn(v)), __bfloat162float(__float2bfloat16_rn(total(tok, j + 8))));
+        if (ACT == 2) v = relu2(v);
+        if (ACT == 3) v = gelu_erf(v);
+        reinterpret_cast<O*>(a.out)[(size_t)s_dst[tok] * a.ldo + col] = from_f32<O>(v);
+    }
+}
+
+// Row tiles of BM pairs that any routing can need: every expert may add one that is not full.
+int most_tiles(const LlmeGroupedArgs& a, int BM) {
+    const int most = a.num_experts < a.pairs ? a.num_experts : a.pairs, tiles = (a.pairs + BM - 1) / BM + most;
+    return tiles < a.pairs ? tiles : a.pairs;
+}
+
+template <int MT, int ACT, typename O>
+int launch_skinny(const LlmeGroupedArgs& a, cudaStream_t s) {
+    const int tiles = most_tiles(a, 8 * MT), cols = ACT == 1 ? 8 : 16, n_out = ACT == 1 ? a.n / 2 : a.n;
+    if (tiles > 65535) LLME_REFUSE("grouped_linear_tc: %d row tiles exceed a launch", tiles);
+    llme_launch(grouped_skinny_kernel<MT, ACT, O>, dim3((n_out + cols - 1) / cols, tiles), dim3(32 * SKINNY_WARPS), 0, s, a);
+    LLME_LAUNCH_STATUS();
+}
+
 template <int BM, int BN, int WM, int WNW, int STAGES, int ACT, typename O>
 int launch(const LlmeGroupedArgs& a, cudaStream_t s) {
     constexpr int SMEM = STAGES * (BM + (ACT == 1 ? 2 : 1) * BN) * LDS * (int)sizeof(bf16);
     const int n_out = ACT == 1 ? a.n / 2 : a.n;
-    const int most = a.num_experts < a.pairs ? a.num_experts : a.pairs;
-    int tiles = (a.pairs + BM - 1) / BM + most;           // every expert may add one tile that is not full
-    if (tiles > a.pairs) tiles = a.pairs;
+    const int tiles = most_tiles(a, BM);
     if (tiles > 65535) {
         snprintf(llme_error_buffer(), 512, "grouped_linear_tc: %d row tiles exceed a launch", tiles);
         return -1;
@@ -217,10 +341,15 @@ int launch(const LlmeGroupedArgs& a, cudaStream_t s) {
     LLME_LAUNCH_STATUS();
 }
 
+// Rows an expert in the mean (the routing itself is on the device): tiles of 8 pairs, of 16, or of 64 through shared memory.  (From 4 rows on
+// the tcgen05 kernel serves what it can; without it 16-pair tiles take that mixture 266 us at 124 tokens and 327 us at 160, 64-pair
+// tiles 279 us at 400.)
+constexpr long long SKINNY_8 = 4, SKINNY_16 = 16;
+
 template <int ACT, typename O>
 int dispatch(const LlmeGroupedArgs& a, cudaStream_t s) {
-    // few rows per expert: tiles of 16 rows, so that little of a tile is padding and every weight is read once
-    if ((long long)a.pairs < 32LL * a.num_experts) return launch<16, 128, 1, 4, 4, ACT, O>(a, s);     // three steps of weights in flight per block
+    if ((long long)a.pairs <= SKINNY_8 * a.num_experts) return launch_skinny<1, ACT, O>(a, s);
+    if ((long long)a.pairs < SKINNY_16 * a.num_experts) return launch_skinny<2, ACT, O>(a, s);
     return launch<64, 64, 1, 4, 3, ACT, O>(a, s);
 }
 
