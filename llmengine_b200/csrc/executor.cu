@@ -974,7 +974,10 @@ int op_moe_route(LlmeExecutor& ex, const LlmeMoeRouteOp& o, const LlmeStep& s, c
     return rc;
 }
 
-constexpr long long GROUPED_ROWS = 64;      // rows an expert gets in the mean, from which on tiles of 128 rows pay
+// Rows an expert gets in the mean, from which on the tcgen05 kernel is ahead: its tiles of 128 rows are mostly padding then, but the
+// experts' matrices are what takes the time, and it reads them once.  A mixture of 4 of 32 experts of 2,048 x 2,048 (bfloat16, whole layer),
+// this kernel against the warp-level ones: 16 tokens (2 rows) 153 / 143 us, 32 (4 rows) 175 / 186, 96 177 / 220, 250 185 / 446, 500 198 / 395.
+constexpr long long GROUPED_ROWS = 4;
 
 int op_grouped_linear(LlmeExecutor& ex, const LlmeGroupedLinearOp& o, const LlmeStep& s, cudaStream_t st) {
     if (s.num_tokens <= 0) return 0;
