@@ -398,26 +398,26 @@ constexpr int DSTAGES = 2;        // stage buffers per warp (one sub-tile in fli
 constexpr int CL_SLOTS = 48;      // (split, row) partial results a cluster's first block can take in its shared memory
 constexpr int STAGE_ELEMS = 2 * SUB * LDS;   // K rows then V rows
 
-// One warp loads keys [j0, j0+16) (K and V) into its stage buffer; keys outside [lo, hi] become zeros.
+// One warp loads keys [j0, j0+16) (K and V) into its stage buffer; keys outside [lo, hi] become zeros, but for the first `kept` ones.
 // When the page size is a multiple of 16 (page_shift >= 4) the 16 keys lie in one page: one look-up in the
 // block table, and every lane's addresses differ from one another only by constants.
 // `bt` points at the entry of block `bt_first` (the request's row of the block table in global memory, or the
 // part of it that the block has copied into shared memory).
 __device__ __forceinline__ void load_sub_tile(bf16* dst, const bf16* cache, const int* bt, int bt_first, int kvh, int nkv, int ps,
-                                              int page_shift, int j0, int lo, int hi) {
+                                              int page_shift, int j0, int lo, int hi, int kept = 0) {
     const int lane = threadIdx.x & 31;
     constexpr int CHUNKS = HD / 8;                 // 16-byte chunks per key row
     constexpr int TOTAL = SUB * CHUNKS;            // chunks of K (and as many of V)
     if (page_shift >= 4) {
         const int blk = j0 >> page_shift;
-        const bool any = j0 + SUB - 1 >= lo && j0 <= hi;
+        const bool any = (j0 + SUB - 1 >= lo || j0 < kept) && j0 <= hi;
         const bf16* kbase = cache;
         if (any) kbase = cache + ((((size_t)bt[blk - bt_first] * 2) * nkv + kvh) * ps + (j0 - (blk << page_shift))) * HD;
         const size_t v_off = (size_t)nkv * ps * HD;
 #pragma unroll
         for (int c = lane; c < TOTAL; c += 32) {
             const int r = c / CHUNKS, ch = c - r * CHUNKS;
-            const bool valid = j0 + r >= lo && j0 + r <= hi;
+            const bool valid = (j0 + r >= lo || j0 + r < kept) && j0 + r <= hi;
             const bf16* src = kbase + r * HD + ch * 8;
             cp_async_16(dst + r * LDS + ch * 8, valid ? src : cache, valid);
             cp_async_16(dst + (SUB + r) * LDS + ch * 8, valid ? src + v_off : cache, valid);
@@ -428,7 +428,7 @@ __device__ __forceinline__ void load_sub_tile(bf16* dst, const bf16* cache, cons
     for (int c = lane; c < TOTAL; c += 32) {
         const int r = c / CHUNKS, ch = c - r * CHUNKS;
         const int j = j0 + r;
-        const bool valid = j >= lo && j <= hi;
+        const bool valid = (j >= lo || j < kept) && j <= hi;
         const bf16* ksrc = cache;
         if (valid) {
             const int blk = page_shift >= 0 ? (j >> page_shift) : (j / ps);
@@ -508,7 +508,12 @@ __device__ __forceinline__ void norm_rotate_head(const bf16* src, const void* ga
     }
 }
 
-__global__ void __launch_bounds__(THREADS) attention_decode_kernel(FastAttnArgs a, FusedQkv f) {
+// Options of other designs, in a form of the kernel of its own (EXT): a logit per head that only joins the denominator, first
+// positions that are seen beside the window, a cap c on the scores (s -> c tanh(s / c) behind the scale).
+struct DecodeExt { const float* sink; int keep_first; float softcap; };
+
+template <bool EXT>
+__global__ void __launch_bounds__(THREADS) attention_decode_kernel(FastAttnArgs a, FusedQkv f, DecodeExt x) {
     // Launched while the kernel before it is still running (programmatic dependent launch), the kernel may read, before
     // pdl_wait(), only what that kernel does not write.  Taking the raw projections (f.qkv), it follows the product
     // that made them: the step's lengths and tables and the keys and values of earlier positions are older than that
@@ -549,12 +554,25 @@ __global__ void __launch_bounds__(THREADS) attention_decode_kernel(FastAttnArgs 
 
     // this block's share of the 16-key sub-tiles, in whole groups of four (one per warp)
     const int sub_first = lo / SUB, sub_last = p / SUB;
-    const int n_groups = (sub_last - sub_first + 4) / 4;
+    // kept first positions: their sub-tiles are numbered in front of the window's
+    const int kept = EXT && a.window > 0 ? min(x.keep_first, lo) : 0, n_kept = EXT ? min((kept + SUB - 1) / SUB, sub_first) : 0;
+    const int n_groups = (n_kept + sub_last - sub_first + 4) / 4;
     const int per = (n_groups + a.splits - 1) / a.splits;
-    const int my_first = sub_first + split * per * 4;
+    const int my_first = sub_first - n_kept + split * per * 4;
+    auto first_key = [&](int sub) { return (EXT && sub < sub_first ? sub - (sub_first - n_kept) : sub) * SUB; };
     const int my_last = min(sub_last, my_first + per * 4 - 1);
 
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};
+    if (EXT && x.sink && split == 0 && (threadIdx.x >> 5) == 0) {     // the sink counts once
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int row = ((threadIdx.x & 31) >> 2) + 8 * i;
+            if (row < rows_here) {
+                m_run[i] = x.sink[kvh * G + g0 + row] * LOG2E;
+                l_run[i] = 1.0f;
+            }
+        }
+    }
     float o[DTILES][4];
 #pragma unroll
     for (int d = 0; d < DTILES; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.0f;
@@ -565,8 +583,8 @@ __global__ void __launch_bounds__(THREADS) attention_decode_kernel(FastAttnArgs 
     __shared__ int page_tab[PAGE_TAB];
     const int* tab = bt;
     int tab_first = 0;
-    if (my_first <= my_last) {
-        const int blk_first = (max(my_first * SUB, lo)) / ps, blk_last = min(my_last * SUB + SUB - 1, p) / ps;
+    if (my_first <= my_last && my_last >= sub_first) {
+        const int start = max(my_first, sub_first) * SUB, blk_first = (EXT && kept > start ? start : max(start, lo)) / ps, blk_last = min(my_last * SUB + SUB - 1, p) / ps;
         if (blk_last - blk_first < PAGE_TAB) {
             for (int i = threadIdx.x; i <= blk_last - blk_first; i += THREADS) page_tab[i] = bt[blk_first + i];
             tab = page_tab;
@@ -574,6 +592,10 @@ __global__ void __launch_bounds__(THREADS) attention_decode_kernel(FastAttnArgs 
             __syncthreads();
         }
     }
+    auto load_sub = [&](bf16* dst, int sub) {
+        const bool front = EXT && sub < sub_first;                   // (in front of the part of the table that was copied)
+        load_sub_tile(dst, a.cache, front ? bt : tab, front ? 0 : tab_first, kvh, a.nkv, ps, page_shift, first_key(sub), lo, p, kept);
+    };
     const float* cs_row = nullptr;
     if (f.qkv && f.cos_sin) {
         const int pos = p < 0 ? 0 : (p >= f.max_positions ? f.max_positions - 1 : p);      // the host refuses such positions
@@ -622,7 +644,7 @@ __global__ void __launch_bounds__(THREADS) attention_decode_kernel(FastAttnArgs 
 #pragma unroll
         for (int st = 0; st < DSTAGES - 1; ++st) {
             const int sub = my_first + warp + 4 * st;
-            if (sub <= my_last) load_sub_tile(mine + st * STAGE_ELEMS, a.cache, tab, tab_first, kvh, a.nkv, ps, page_shift, sub * SUB, lo, p);
+            if (sub <= my_last) load_sub(mine + st * STAGE_ELEMS, sub);
             cp_async_commit();
         }
         if (!waited) pdl_wait();           // the first key/value loads are under way: now the projections
@@ -652,13 +674,13 @@ __global__ void __launch_bounds__(THREADS) attention_decode_kernel(FastAttnArgs 
         int plo[2] = {lo, lo}, phi[2];
         phi[0] = (lane >> 2) < rows_here ? p : -1;
         phi[1] = (lane >> 2) + 8 < rows_here ? p : -1;
-        const float sc = a.scale * LOG2E;
+        const bool capped = EXT && x.softcap > 0.0f;
+        const float to_cap = capped ? a.scale / x.softcap : 0.0f;
+        const float sc = (capped ? x.softcap : a.scale) * LOG2E;            // (behind the cap a score is tanh(.))
         int n = 0;
         for (int sub = my_first + warp; sub <= my_last; sub += 4, ++n) {
             const int ahead = sub + 4 * (DSTAGES - 1);
-            if (ahead <= my_last)
-                load_sub_tile(mine + ((n + DSTAGES - 1) % DSTAGES) * STAGE_ELEMS, a.cache, tab, tab_first, kvh, a.nkv, ps, page_shift,
-                              ahead * SUB, lo, p);
+            if (ahead <= my_last) load_sub(mine + ((n + DSTAGES - 1) % DSTAGES) * STAGE_ELEMS, ahead);
             cp_async_commit();
             cp_async_wait<DSTAGES - 1>();                   // this lane's copies of sub-tile n are done
             __syncwarp();                                   // ... and so are the other lanes'
@@ -667,10 +689,22 @@ __global__ void __launch_bounds__(THREADS) attention_decode_kernel(FastAttnArgs 
             qk_tile<2>(sreg, qf, Kt, 0);
             // only the sub-tiles at the two ends of the visible range hold keys that must be masked
             // (rows past the group's heads hold zero queries: finite, and never stored)
-            if (sub * SUB >= lo && sub * SUB + SUB - 1 <= p)
-                softmax_update<2, false>(sreg, m_run, l_run, o, sub * SUB, plo, phi, sc);
+            const int j0 = first_key(sub);
+            if (EXT) {
+                const bool all = j0 >= lo && j0 + SUB - 1 <= p;
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        if (capped) sreg[nt][c] = tanhf(sreg[nt][c] * to_cap);
+                        const int j = j0 + nt * 8 + (lane & 3) * 2 + (c & 1);
+                        if (!all && (j > p || (j < lo && j >= kept))) sreg[nt][c] = -INFINITY;
+                    }
+                softmax_update<2, false>(sreg, m_run, l_run, o, j0, plo, phi, sc);
+            } else if (j0 >= lo && j0 + SUB - 1 <= p)
+                softmax_update<2, false>(sreg, m_run, l_run, o, j0, plo, phi, sc);
             else
-                softmax_update<2, true>(sreg, m_run, l_run, o, sub * SUB, plo, phi, sc);
+                softmax_update<2, true>(sreg, m_run, l_run, o, j0, plo, phi, sc);
             pv_tile<2>(o, sreg, Kt + SUB * LDS, 0);
             __syncwarp();                                   // all lanes have read the stage before it is refilled
         }
@@ -885,7 +919,7 @@ LLME_API int llme_attention_decode_clusters(int splits) {
     if (splits < 2 || splits > 8) return 0;
     static int known[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     if (known[splits]) return known[splits];
-    if (cudaFuncSetAttribute(attention_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DECODE_SMEM) != cudaSuccess) {
+    if (cudaFuncSetAttribute(attention_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DECODE_SMEM) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -901,7 +935,7 @@ LLME_API int llme_attention_decode_clusters(int splits) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, attention_decode_kernel, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, attention_decode_kernel<false>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -927,14 +961,15 @@ LLME_API int llme_attention_portion(const FastAttnArgs* args, int max_q_len, cud
     LLME_LAUNCH_STATUS();
 }
 
-static int launch_decode(const FastAttnArgs& a, const FusedQkv& f, cudaStream_t stream) {
+template <bool EXT>
+static int launch_decode(const FastAttnArgs& a, const FusedQkv& f, const DecodeExt& x, cudaStream_t stream) {
     if (a.n_rows <= 0) return 0;
     if (int rc = check_common(a, f.qkv != nullptr)) return rc;
     if (a.splits < 1 || a.splits > 1024) LLME_REFUSE("attention: splits must be in 1..1024, got %d", a.splits);
     if (a.splits > 1 && !a.scratch) LLME_REFUSE("attention: split decoding needs scratch memory");
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DECODE_SMEM);
+        cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel<EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DECODE_SMEM);
         if (e != cudaSuccess) LLME_REFUSE("attention: cannot reserve %zu bytes of shared memory: %s", DECODE_SMEM, cudaGetErrorString(e));
         configured = true;
     }
@@ -964,16 +999,22 @@ static int launch_decode(const FastAttnArgs& a, const FusedQkv& f, cudaStream_t 
         attr[1].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 2;
-        cudaLaunchKernelEx(&cfg, attention_decode_kernel, a, f);
+        cudaLaunchKernelEx(&cfg, attention_decode_kernel<EXT>, a, f, x);
         LLME_LAUNCH_STATUS();
     }
-    llme_launch(attention_decode_kernel, dim3(grid), dim3(THREADS), DECODE_SMEM, stream, a, f);
+    llme_launch(attention_decode_kernel<EXT>, dim3(grid), dim3(THREADS), DECODE_SMEM, stream, a, f, x);
     LLME_LAUNCH_STATUS();
 }
 
 LLME_API int llme_attention_decode(const FastAttnArgs* args, cudaStream_t stream) {
     const FusedQkv none = {};
-    return launch_decode(*args, none, stream);
+    return launch_decode<false>(*args, none, DecodeExt{}, stream);
+}
+
+// The same with a sink (32-bit [nh] or null), kept first positions and a cap on the scores (0: none).
+LLME_API int llme_attention_decode_ext(const FastAttnArgs* args, const float* sink, int keep_first, float softcap, cudaStream_t stream) {
+    const FusedQkv none = {};
+    return launch_decode<true>(*args, none, DecodeExt{sink, keep_first, softcap}, stream);
 }
 
 // The same with the raw q|k|v projections of the new tokens instead of finished queries (args->q is ignored):
@@ -988,5 +1029,5 @@ LLME_API int llme_attention_decode_fused(const FastAttnArgs* args, const FusedQk
     if ((f.q_gain == nullptr) != (f.k_gain == nullptr)) LLME_REFUSE("attention: the fused decode norms both queries and keys or neither");
     if (f.q_gain && f.gain_dtype != LLME_F32 && f.gain_dtype != LLME_BF16) LLME_REFUSE("attention: unsupported gain dtype %d", f.gain_dtype);
     if (f.cos_sin && f.max_positions <= 0) LLME_REFUSE("attention: rotation needs the table's length");
-    return launch_decode(*args, f, stream);
+    return launch_decode<false>(*args, f, DecodeExt{}, stream);
 }

@@ -37,6 +37,7 @@ typedef int (*AttnPlainFn)(const LlmeAttnArgs*, int, cudaStream_t);
 typedef int (*AttnPortionFn)(const LlmeFastAttnArgs*, int, cudaStream_t);
 typedef int (*AttnDecodeFn)(const LlmeFastAttnArgs*, cudaStream_t);
 typedef int (*AttnDecodeFusedFn)(const LlmeFastAttnArgs*, const LlmeFusedQkv*, cudaStream_t);
+typedef int (*AttnDecodeExtFn)(const LlmeFastAttnArgs*, const float*, int, float, cudaStream_t);
 typedef long long (*AttnScratchFn)(int, int, int);
 typedef int (*AttnTcFn)(const void*, long long, long long, const LlmeTcAttnArgs*, int, cudaStream_t);
 typedef const char* (*LastErrorFn)();
@@ -827,7 +828,20 @@ int window_attend(LlmeExecutor& ex, const LlmeWindowAttentionOp& o, const LlmeSt
             f.rows = s.portion_rows; f.n_rows = s.num_portion;
             if (int rc = ex.launched(tc(&f, s.max_portion_len, 0, st), "window_attention_tc")) return rc;
         }
-        if (s.num_decode > 0) {
+        // single tokens likewise: the split-context kernel with those options (34 requests of 32 / 8 heads of 128, 800 keys: 23 us against 71 us of
+        // the warp-level kernel and its merge)
+        auto* ext = o.dk == o.dv && o.value_share <= 1 ? (AttnDecodeExtFn)ex.find_hd("attention_decode_ext", o.dk) : nullptr;
+        const long long pairs = (long long)s.num_decode * o.nkv * ((rep + 15) / 16);             // (request, key/value head, 16 query heads)
+        if (s.num_decode > 0 && ext && o.decode_scratch && pairs <= 65535 && s.num_decode <= 65535 && fast_attention(ex, o.dtype, o.dk) &&
+            aligned16(o.q, o.cache, o.out)) {
+            LlmeAttendOp at = {o.q, o.out, o.dtype, o.cache, o.cache_pages * 2 * o.nkv * ps, o.group, o.nh, o.nkv, o.dk, o.window, o.scale,
+                               o.decode_scratch, o.decode_scratch_floats};
+            const int splits = decode_splits(ex, s.num_decode, o.nh, o.nkv, o.dk, o.window, s.max_decode_ctx);
+            if (int rc = scratch_check(ex, at, s.num_decode, splits)) return rc;
+            LlmeFastAttnArgs d = {};
+            fill_fast(d, at, s, s.decode_rows, s.num_decode, splits);
+            if (int rc = ex.launched(ext(&d, o.sink, o.keep_first, o.softcap, st), "attention_decode_ext")) return rc;
+        } else if (s.num_decode > 0) {
             f.rows = s.decode_rows; f.n_rows = s.num_decode;
             // key ranges: enough blocks for two an SM, no range shorter than two chunks of 64 keys, at most 8
             long long keys = s.max_decode_ctx;

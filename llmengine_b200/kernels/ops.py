@@ -224,6 +224,7 @@ class CudaOps:
         "attention_plain": {"attention_plain": "llme_attention_plain"},
         "attention_fast": {"attention_portion/{hd}": "llme_attention_portion", "attention_decode/{hd}": "llme_attention_decode",
                            "attention_decode_fused/{hd}": "llme_attention_decode_fused",
+                           "attention_decode_ext/{hd}": "llme_attention_decode_ext",
                            "attention_decode_scratch/{hd}": "llme_attention_decode_scratch_floats",
                            "attention_decode_clusters/{hd}": "llme_attention_decode_clusters"},
         "attention_tc": {"attention_tc/{hd}": "llme_attention_tc"},
@@ -273,10 +274,12 @@ class CudaOps:
                         if (a["qk_dim"], a["v_dim"]) == (64, 128) and self.chosen("attention.portion") == "tcgen05":
                             want("attention_tc@HEAD_DIM=64,VALUE_DIM=128,MAPS=2")
                 if fast_attention and a.get("decode_scratch") is not None and self.fast_attention_supports(a["qk_dim"], a["q"].dtype):
-                    want(f"attention_fast@HEAD_DIM={a['qk_dim']}")       # ordinary attention: the grouped-query kernels
+                    want(f"attention_fast@HEAD_DIM={a['qk_dim']}")       # keys and values of one width: the grouped-query kernels
                     if a["qk_dim"] in (64, 128) and self.chosen("attention.portion") == "tcgen05":
                         want(f"attention_tc@HEAD_DIM={a['qk_dim']}")
-                elif fast_attention and build.has_source("attention_window_tc") and self.window_tc_supports(a["qk_dim"], a["v_dim"], a["q"].dtype):
+                plain_mask = not (a["keep_first"] or a.get("sink") is not None or a.get("softcap"))
+                if (fast_attention and build.has_source("attention_window_tc") and self.window_tc_supports(a["qk_dim"], a["v_dim"], a["q"].dtype)
+                        and not (plain_mask and a.get("decode_scratch") is not None and self.fast_attention_supports(a["qk_dim"], a["q"].dtype))):
                     want(f"attention_window_tc@DK={a['qk_dim']},DV={a['v_dim']}")
                     if a["qk_dim"] == a["v_dim"] and a["qk_dim"] in (64, 128) and a.get("value_share", 1) <= 1 and self.chosen("attention.portion") == "tcgen05":
                         want(f"attention_tc@HEAD_DIM={a['qk_dim']}")

@@ -329,9 +329,10 @@ class WindowSinkAttention(Part):
             keep_first=self.keep_first, scale=self.scale, sink=self.sink,
             q_bias=self.q_bias, k_bias=self.k_bias, v_bias=self.v_bias, head_norm=self.head_norm, softcap=self.softcap,
             interleaved=bool(pos is not None and getattr(pos, "interleaved", False)),
-            # an ordinary causal softmax over keys and values of one width: the kernels of plain grouped-query attention serve it
+            # keys and values of one width: the kernels of plain grouped-query attention serve an ordinary causal softmax, and for
+            # heads of 64 or 128 also one with a sink, kept first positions or a cap
             decode_scratch=(rt.attention_scratch(self.nh, self.nkv, self.dk)
-                            if rt.dtype == torch.bfloat16 and self.ordinary else None),
+                            if rt.dtype == torch.bfloat16 and (self.ordinary or (self.dk == self.dv and self.dk in (64, 128))) else None),
             # up to 8 key ranges per decoded token: a maximum, a sum and an output row per range and head
             scratch=(rt.buffer("window_attention_scratch", 1, rt.max_requests * self.nh * 8 * (self.dv + 2), torch.float32,
                                exact=True).view(-1) if rt.dtype == torch.bfloat16 else None))
