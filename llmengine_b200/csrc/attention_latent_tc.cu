@@ -10,8 +10,9 @@
 //      bfloat16 in shared memory,
 //   3. share the outputs: warp (rg, wg) adds P V for its 16 rows and its RANK/WG columns, V being the first RANK
 //      values of the same key rows (ldmatrix.trans), so nothing is loaded twice.
-// Keys arrive through a two-stage cp.async pipeline, page by page through the block table; rows outside the
-// needed range are zero-filled, never read.  The running maximum of a row starts at its head's sink (and the
+// Keys arrive two tiles ahead at most, one bulk copy per row (a row of the cache is contiguous; sixteen-byte copies by all threads were a
+// quarter of the kernel's instructions), page by page through the block table; rows outside the needed range are zero-filled, never
+// read.  The wait for a tile is bounded: one that gives up sets the error flag (llme_latent_attention_tc_status()).  The running maximum of a row starts at its head's sink (and the
 // running sum at one) when the mixer has one.  With a window W a query sees only the last W keys: a tile's walk starts
 // at the tile that holds the nearest key any of its rows sees.  A decode step may split the keys of a request over several blocks,
 // whose partial sums meet in scratch memory and are merged by a second kernel.
@@ -55,6 +56,19 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
 
+constexpr unsigned WAIT_LIMIT = 1u << 20;          // polls (each may suspend for a while): far beyond any legitimate wait
+__device__ int g_status = 0;                       // 1: a wait gave up
+
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) {
+    for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
+        unsigned ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
 struct Args {
     const __nv_bfloat16* q; const __nv_bfloat16* cache; __nv_bfloat16* out;
     const float* sink;
@@ -66,7 +80,7 @@ struct Args {
 };
 
 // RG groups of 16 query rows, WG = 8 / RG warps per group, key tiles of BN.
-template <int RG, int BN, int STAGES>
+template <int RG, int BN>
 __global__ void __launch_bounds__(WARPS * 32, RG <= 2 && RANK <= 320 ? 2 : 1) latent_attention_tc_kernel(Args a) {
     constexpr int WG = WARPS / RG, BM = 16 * RG;
     constexpr int KW = BN / WG, NT_S = KW / 8;             // keys and 8-key tiles of a warp's share of the scores
@@ -76,10 +90,11 @@ __global__ void __launch_bounds__(WARPS * 32, RG <= 2 && RANK <= 320 ? 2 : 1) la
     const int width = RANK + a.rot, widthp = (width + 63) & ~63, ld = widthp + 8;      // whole groups of four 16-wide steps
     __nv_bfloat16* q_s = (__nv_bfloat16*)smem_raw;                       // [BM][ld]
     __nv_bfloat16* k_s = q_s + (size_t)BM * ld;                          // [2][BN][ld]
-    __nv_bfloat16* p_s = k_s + (size_t)STAGES * BN * ld;                 // [BM][BN + 8]
+    __nv_bfloat16* p_s = k_s + (size_t)2 * BN * ld;                 // [BM][BN + 8]
     float* red = (float*)(p_s + (size_t)BM * (BN + 8));                  // [WG][BM]
     int* page_s = (int*)(red + WG * BM);                                 // [PAGES]
     constexpr int LDP = BN + 8;
+    __shared__ unsigned long long key_bar[2];                            // a tile's rows have landed in stage 0 / 1
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rg = warp % RG, wg = warp / RG;
@@ -106,8 +121,8 @@ __global__ void __launch_bounds__(WARPS * 32, RG <= 2 && RANK <= 320 ? 2 : 1) la
     const int ps_shift = (ps & (ps - 1)) == 0 ? __ffs(ps) - 1 : -1;
     auto page_of = [&](int j) { return ps_shift >= 0 ? j >> ps_shift : j / ps; };
     // The pages of this block's keys, looked up once: a look-up per row in front of its copies, one after the other, took longer than
-    // the copies (24 requests of 16 heads over 4,000 keys: 54 us, 41 us
-    // without, and with the queries kept in registers).
+    // the copies (24 requests of 16 heads over 4,000 keys: 54 us; 41 us
+    // without, and with the queries kept in registers; 32 us with one copy a row).
     const int j_first = max(kmin, t_begin * BN), j_last = min(pmax, t_end * BN - 1);
     const int page0 = page_of(j_first), held = j_last >= j_first ? page_of(j_last) - page0 + 1 : 0;
     const bool in_table = held <= PAGES;
@@ -115,30 +130,38 @@ __global__ void __launch_bounds__(WARPS * 32, RG <= 2 && RANK <= 320 ? 2 : 1) la
     // the padding columns of Q and of both key stages are zero for the whole kernel
     if (widthp > width) {
         const int pad = widthp - width;
-        for (int e = tid; e < (BM + STAGES * BN) * pad; e += blockDim.x) {
+        for (int e = tid; e < (BM + 2 * BN) * pad; e += blockDim.x) {
             const int row = e / pad, c = width + e % pad;
             (row < BM ? q_s + (size_t)row * ld : k_s + (size_t)(row - BM) * ld)[c] = __float2bfloat16(0.0f);
         }
+    }
+    if (tid == 0) {
+        for (int s = 0; s < 2; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&key_bar[s])));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     pdl_wait();
     if (in_table)
         for (int i = tid; i < held; i += blockDim.x) page_s[i] = bt[page0 + i];
     __syncthreads();
 
-    // A warp brings whole key rows, the lanes share a row's 16-byte pieces.
+    // Eight lanes of every warp request a row each (or four: a copy takes its warp some 100 cycles to issue); rows that no query of the block sees are written as zeros by everybody.
     auto load_keys = [&](int tile, int stage) {
         __nv_bfloat16* dst = k_s + (size_t)stage * BN * ld;
-        const int j0 = tile * BN;
-        for (int kr = warp; kr < BN; kr += WARPS) {
-            const int j = j0 + kr;
-            __nv_bfloat16* d = dst + (size_t)kr * ld;
-            if (j <= pmax && j >= kmin) {                        // (a page the window has passed may be gone: never read)
-                const int blk = page_of(j), page = in_table ? page_s[blk - page0] : bt[blk];
-                const __nv_bfloat16* src = a.cache + ((size_t)page * ps + (j - blk * ps)) * width;
-                for (int c = lane; c < chunks; c += 32) cp_async16(d + c * 8, src + c * 8);
-            } else {
-                for (int c = lane; c < chunks; c += 32) *reinterpret_cast<uint4*>(d + c * 8) = make_uint4(0u, 0u, 0u, 0u);
-            }
+        const int j0 = tile * BN, from = max(j0, kmin), to = min(j0 + BN - 1, pmax);
+        if (to - from < BN - 1) {
+            for (int kr = warp; kr < BN; kr += WARPS)
+                if (j0 + kr < from || j0 + kr > to)
+                    for (int c = lane; c < chunks; c += 32) *reinterpret_cast<uint4*>(dst + (size_t)kr * ld + c * 8) = make_uint4(0u, 0u, 0u, 0u);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // a copy that later goes to these rows comes behind the zeros
+        }
+        if (tid == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&key_bar[stage])), "r"((unsigned)((to - from + 1) * width * 2)) : "memory");
+        const int j = j0 + warp * (BN / WARPS) + lane, kr = j - j0;
+        if (lane < BN / WARPS && j >= from && j <= to) {         // (a page the window has passed may be gone: never read)
+            const int blk = page_of(j), page = in_table ? page_s[blk - page0] : bt[blk];
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(smem_u32(dst + (size_t)kr * ld)), "l"(a.cache + ((size_t)page * ps + (j - blk * ps)) * width), "r"((unsigned)(width * 2)),
+                           "r"(smem_u32(&key_bar[stage])) : "memory");
         }
     };
 
@@ -154,12 +177,9 @@ __global__ void __launch_bounds__(WARPS * 32, RG <= 2 && RANK <= 320 ? 2 : 1) la
             }
         }
     }
-    if (t_begin < t_end) load_keys(t_begin, 0);
     cp_async_commit();
-    if (STAGES == 2) {                             // the second tile is requested at once, not when the first has landed
-        if (t_begin + 1 < t_end) load_keys(t_begin + 1, 1);
-        cp_async_commit();
-    }
+    if (t_begin < t_end) load_keys(t_begin, 0);
+    if (t_begin + 1 < t_end) load_keys(t_begin + 1, 1);          // the second tile is requested at once, not when the first has landed
 
     // this thread's two rows of its group: lane / 4 and lane / 4 + 8
     const int lr0 = rg * 16 + (lane >> 2), lr1 = lr0 + 8;
@@ -182,15 +202,14 @@ __global__ void __launch_bounds__(WARPS * 32, RG <= 2 && RANK <= 320 ? 2 : 1) la
     uint32_t qk[Q_STEPS > 0 ? Q_STEPS : 1][4];
 
     for (int tile = t_begin; tile < t_end; ++tile) {
-        const int stage = STAGES == 1 ? 0 : (tile - t_begin) & 1;
-        if (STAGES == 1 && tile > t_begin) {
-            __syncthreads();                       // everyone has finished with the tile before this one
-            load_keys(tile, 0);
-            cp_async_commit();
+        const int stage = (tile - t_begin) & 1;
+        cp_async_wait<0>();                        // (the queries, before the first tile)
+        const bool landed = mbar_wait(&key_bar[stage], (unsigned)((tile - t_begin) >> 1) & 1u);
+        if (__syncthreads_or(!landed)) {           // gave up (the whole block): what is in flight lands, then it leaves
+            if (tid == 0) atomicCAS(&g_status, 0, 1);
+            for (int i = 0; i < 200; ++i) __nanosleep(5000);
+            return;
         }
-        if (STAGES == 2) cp_async_wait<1>();       // everything but the newest request: this tile has landed
-        else cp_async_wait<0>();
-        __syncthreads();
         const __nv_bfloat16* kt = k_s + (size_t)stage * BN * ld;
 
         // 1. scores of this warp's rows against its share of the tile's keys
@@ -228,8 +247,10 @@ __global__ void __launch_bounds__(WARPS * 32, RG <= 2 && RANK <= 320 ? 2 : 1) la
             }
         } else {
             const uint32_t k_addr = smem_u32(kt + (size_t)(wg * KW + (lane & 7)) * ld + ((lane >> 3) & 1) * 8);
-            // one 8-key tile: two accumulators (even and odd steps) keep two products in flight, added at the end
-            float s2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            // one 8-key tile: four accumulators keep four products in flight, added at the end
+            float s2[3][4];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) s2[i][0] = s2[i][1] = s2[i][2] = s2[i][3] = 0.0f;
             if (Q_STEPS > 0 && q_kept) {
 #pragma unroll
                 for (int ks = 0; ks < Q_STEPS; ks += 4) {
@@ -238,7 +259,7 @@ __global__ void __launch_bounds__(WARPS * 32, RG <= 2 && RANK <= 320 ? 2 : 1) la
 #pragma unroll
                         for (int u = 0; u < 4; ++u) ldmatrix_x2(k_addr + (ks + u) * 32, kb[u][0], kb[u][1]);
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) mma_bf16((u & 1) ? s2 : s[0], qk[ks + u][0], qk[ks + u][1], qk[ks + u][2], qk[ks + u][3], kb[u][0], kb[u][1]);
+                        for (int u = 0; u < 4; ++u) mma_bf16(u ? s2[u > 0 ? u - 1 : 0] : s[0], qk[ks + u][0], qk[ks + u][1], qk[ks + u][2], qk[ks + u][3], kb[u][0], kb[u][1]);
                     }
                 }
             } else
@@ -250,10 +271,10 @@ __global__ void __launch_bounds__(WARPS * 32, RG <= 2 && RANK <= 320 ? 2 : 1) la
                     ldmatrix_x2(k_addr + (ks + u) * 32, kb[u][0], kb[u][1]);
                 }
 #pragma unroll
-                for (int u = 0; u < 4; ++u) mma_bf16((u & 1) ? s2 : s[0], qa[u][0], qa[u][1], qa[u][2], qa[u][3], kb[u][0], kb[u][1]);
+                for (int u = 0; u < 4; ++u) mma_bf16(u ? s2[u > 0 ? u - 1 : 0] : s[0], qa[u][0], qa[u][1], qa[u][2], qa[u][3], kb[u][0], kb[u][1]);
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) s[0][i] += s2[i];
+            for (int i = 0; i < 4; ++i) s[0][i] = (s[0][i] + s2[0][i]) + (s2[1][i] + s2[2][i]);
         }
         // 2. scale, mask, row maxima over the whole tile
         float t0 = -INFINITY, t1 = -INFINITY;
@@ -327,11 +348,8 @@ __global__ void __launch_bounds__(WARPS * 32, RG <= 2 && RANK <= 320 ? 2 : 1) la
                 mma_bf16(o[NT_O - 1], a0, a1, a2, a3, b0, b1);
             }
         }
-        if (STAGES == 2) {                         // the stage is free again: the tile after the next one goes there
-            __syncthreads();
-            if (tile + 2 < t_end) load_keys(tile + 2, stage);
-            cp_async_commit();
-        }
+        __syncthreads();                           // the stage is free again: the tile after the next one goes there
+        if (tile + 2 < t_end) load_keys(tile + 2, stage);
     }
     cp_async_wait<0>();
 
@@ -419,18 +437,18 @@ __global__ void latent_merge_kernel(const float* __restrict__ scratch, __nv_bflo
     }
 }
 
-template <int RG, int BN, int STAGES = 2>
+template <int RG, int BN>
 size_t smem_bytes(int rot) {
     const int widthp = (RANK + rot + 63) & ~63, ld = widthp + 8, BM = 16 * RG;
-    return ((size_t)BM * ld + (size_t)STAGES * BN * ld + (size_t)BM * (BN + 8)) * 2 + (size_t)(WARPS / RG) * BM * 4 + PAGES * sizeof(int);
+    return ((size_t)BM * ld + (size_t)2 * BN * ld + (size_t)BM * (BN + 8)) * 2 + (size_t)(WARPS / RG) * BM * 4 + PAGES * sizeof(int);
 }
 
-template <int RG, int BN, int STAGES = 2>
+template <int RG, int BN>
 int launch(const Args& a, int n_list, int max_q_len, cudaStream_t stream) {
-    const size_t smem = smem_bytes<RG, BN, STAGES>(a.rot);
+    const size_t smem = smem_bytes<RG, BN>(a.rot);
     static size_t allowed = 0;
     if (smem > allowed) {
-        if (cudaFuncSetAttribute(latent_attention_tc_kernel<RG, BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        if (cudaFuncSetAttribute(latent_attention_tc_kernel<RG, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             cudaGetLastError();
             LLME_REFUSE("latent attention: rows of %d values need %zu bytes of shared memory", RANK + a.rot, smem);
         }
@@ -438,11 +456,18 @@ int launch(const Args& a, int n_list, int max_q_len, cudaStream_t stream) {
     }
     const int BM = 16 * RG;
     dim3 grid(((long long)max_q_len * a.nh + BM - 1) / BM, n_list, a.splits);
-    llme_launch(latent_attention_tc_kernel<RG, BN, STAGES>, grid, dim3(WARPS * 32), smem, stream, a);
+    llme_launch(latent_attention_tc_kernel<RG, BN>, grid, dim3(WARPS * 32), smem, stream, a);
     LLME_LAUNCH_STATUS();
 }
 
 }  // namespace
+
+// 0 if no bounded wait ever gave up (synchronises the device).
+LLME_API int llme_latent_attention_tc_status() {
+    int v = 0;
+    if (cudaMemcpyFromSymbol(&v, g_status, sizeof(int)) != cudaSuccess) return -1;
+    return v;
+}
 
 // Whether rows of RANK + rot values fit the kernel (shared memory of the wider configuration).
 LLME_API int llme_latent_attention_tc_fits(int rot) {

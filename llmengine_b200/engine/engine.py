@@ -433,6 +433,8 @@ class Engine:
         for key in libs:
             if key.startswith("attention_tc@HEAD_DIM="):
                 status = status or int(libs[key].llme_attention_tc_status())
+            if key.startswith("attention_latent_tc@"):
+                status = status or int(libs[key].llme_latent_attention_tc_status())
             if key.startswith("attention_latent_tcgen05@"):
                 status = status or int(libs[key].llme_latent_pair_status())
         if status:
