@@ -13,8 +13,8 @@
 // 16 x 16 threads hold TM x TN outputs each, as packed pairs of neighbouring columns (fma.rn.f32x2: one instruction, each half
 // rounds as fmaf does); operands lie in shared memory k by k, two stages, the next one on its way through registers.
 // Bound by the multiply-adds: 300 x 11008 x 2048 takes 376 us and 300 x 2048 x 5504 216 us (36 and 31 TFLOP/s of 74; 2,048 rows: 50
-// and 44); one block per 64 x 64 tile with 4 x 4 outputs a thread, whatever the shape, took 675 and 617 us.  One row: 117 and 66 us
-// against 275 and 616 us.
+// and 44); one block per 64 x 64 tile with 4 x 4 outputs a thread, whatever the shape, took 675 and 617 us.
+// Up to 32 rows a third form streams the weights (further down).
 //
 // Reference counterparts: sgemm_nt_kernel (src/runtime/kernels/cuda_kernels.cu:282-294,
 // one thread per output, no tiling) and the cublasSgemm call of sgemm_nt_cublas (:892-908).
@@ -243,6 +243,121 @@ int launch(const Problem<WT>& g, int batch, cudaStream_t stream) {
     LLME_LAUNCH_STATUS();
 }
 
+__device__ __forceinline__ float4 load4_shared(const unsigned char* p, float) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4_shared(const unsigned char* p, __nv_bfloat16) { return load4(reinterpret_cast<const __nv_bfloat16*>(p)); }
+// `bytes` of SIZE from src, zeros behind them
+template <int SIZE>
+__device__ __forceinline__ void copy_async(unsigned char* dst, const void* src, int bytes) {
+    const unsigned at = (unsigned)__cvta_generic_to_shared(dst);
+    if (SIZE == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at), "l"(src), "r"(bytes) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(at), "l"(src), "r"(bytes) : "memory");
+}
+
+// A few rows: the weights are streamed.  A block serves 16 weight rows and MT rows of A; each of its warps walks one segment of K,
+// 32 values at a time, through copies of its own (no barrier until the segments are added, in their order).  A lane has R weight
+// rows and T rows of A, and each of its outputs is one chain of multiply-adds in the order of k, as in the tiles.
+// One row is bound by the weights and the chains' latency, 16 rows by the warps' issue (16 weight rows a block is what gives 2,048
+// outputs enough blocks).  Against the tiles, whose steps of 16 values each wait for a barrier (11008 x 2048 / 2048 x 5504, us):
+// 1 row 21 / 19 and 117 / 66, 8 rows 31 / 25 and 117 / 66, 16 rows 45 / 35 and 118 / 67, 32 rows 73 / 50 and 119 / 74.
+constexpr int FEW_N = 16, FEW_K = 32, FEW_ROWS = 32;
+__host__ __device__ constexpr int few_stages(int mt) { return mt <= 4 ? 6 : mt <= 16 ? 5 : 4; }
+template <typename WT, int MT>
+__host__ __device__ constexpr int few_stage_bytes() { return FEW_N * FEW_K * (int)sizeof(WT) + MT * FEW_K * 4; }
+
+template <typename WT, int MT>
+__global__ void gemm_few_f32_kernel(Problem<WT> g) {
+    constexpr int R = MT <= 4 ? 1 : MT <= 16 ? 2 : 4, RG = FEW_N / R, TG = 32 / RG, T = MT / TG;     // a lane's R x T outputs
+    constexpr int STAGES = few_stages(MT), WB = FEW_N * FEW_K * (int)sizeof(WT), STAGE = few_stage_bytes<WT, MT>();
+    constexpr int PIECE = 4 * (int)sizeof(WT);             // four weights
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rg = lane % RG, tg = lane / RG;
+    const float* A = g.A + (size_t)blockIdx.z * g.sa;
+    const WT* W = g.W + (size_t)blockIdx.z * g.sw;
+    float* C = g.C + (size_t)blockIdx.z * g.sc;
+    const int n0 = blockIdx.x * FEW_N, m0 = blockIdx.y * MT;
+    const int k_begin = warp * g.segment, k_end = min(g.K, k_begin + g.segment), chunks = (k_end - k_begin + FEW_K - 1) / FEW_K;
+    unsigned char* mine = smem_raw + (size_t)warp * STAGES * STAGE;
+    // where a row's p-th four values lie: the lanes of one shared-memory pass (8 of 16 bytes, 16 of 8) meet every bank once
+    auto place_w = [](int r, int p) { return (r * 8 + (p ^ ((sizeof(WT) == 4 ? r : r >> 1) & 7))) * PIECE; };
+    auto place_a = [](int r, int p) { return (r * 8 + (p ^ (r & 7))) * 16; };
+    auto request = [&](int c, int stage) {
+        if (c < chunks) {
+            unsigned char* at = mine + stage * STAGE;
+            const int k0 = k_begin + c * FEW_K + (lane & 7) * 4, some = max(0, min(4, k_end - k0));
+#pragma unroll
+            for (int i = 0; i < FEW_N / 4; ++i) {
+                const int r = i * 4 + (lane >> 3), n = n0 + r < g.N ? some : 0;
+                copy_async<PIECE>(at + place_w(r, lane & 7), n ? W + (size_t)(n0 + r) * g.ldw + k0 : W, n * (int)sizeof(WT));
+            }
+#pragma unroll
+            for (int i = 0; i < (MT + 3) / 4; ++i) {
+                const int r = i * 4 + (lane >> 3), n = m0 + r < g.M ? some : 0;
+                if (r < MT) copy_async<16>(at + WB + place_a(r, lane & 7), n ? A + (size_t)(m0 + r) * g.lda + k0 : A, n * 4);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[R][T];
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int t = 0; t < T; ++t) acc[i][t] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < STAGES - 1; ++c) request(c, c);
+    int stage = 0;
+    for (int c = 0; c < chunks; ++c) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncwarp();                                      // every lane's copies are there, and the stage before this one is read
+        request(c + STAGES - 1, stage == 0 ? STAGES - 1 : stage - 1);
+        const unsigned char* at = mine + stage * STAGE;
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+            float4 w[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) w[i] = load4_shared(at + place_w(rg + i * RG, p), WT());
+#pragma unroll
+            for (int t = 0; t < T; ++t) {
+                const float4 v = *reinterpret_cast<const float4*>(at + WB + place_a(tg + t * TG, p));
+#pragma unroll
+                for (int i = 0; i < R; ++i) acc[i][t] = fmaf(v.w, w[i].w, fmaf(v.z, w[i].z, fmaf(v.y, w[i].y, fmaf(v.x, w[i].x, acc[i][t]))));
+            }
+        }
+        stage = stage == STAGES - 1 ? 0 : stage + 1;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    float* part = reinterpret_cast<float*>(mine);          // [MT][16], this segment's sums
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int t = 0; t < T; ++t) part[(tg + t * TG) * FEW_N + rg + i * RG] = acc[i][t];
+    __syncthreads();
+    for (int e = threadIdx.x; e < MT * FEW_N; e += blockDim.x) {
+        const int m = m0 + e / FEW_N, n = n0 + e % FEW_N;
+        if (m >= g.M || n >= g.N) continue;
+        float sum = 0.0f;
+        for (int from = 0; from < g.segments; ++from) {
+            const float v = reinterpret_cast<const float*>(smem_raw + (size_t)from * STAGES * STAGE)[e];
+            sum = from == 0 ? v : sum + v;
+        }
+        C[(size_t)m * g.ldc + n] = sum;
+    }
+}
+
+template <typename WT, int MT>
+int launch_few(const Problem<WT>& g, int batch, cudaStream_t stream) {
+    constexpr int one = few_stages(MT) * few_stage_bytes<WT, MT>();
+    auto kernel = gemm_few_f32_kernel<WT, MT>;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SEGMENTS * one);
+        if (e != cudaSuccess) LLME_REFUSE("gemm_f32: cannot reserve %d bytes of shared memory: %s", MAX_SEGMENTS * one, cudaGetErrorString(e));
+        configured = true;
+    }
+    kernel<<<dim3((g.N + FEW_N - 1) / FEW_N, (g.M + MT - 1) / MT, batch), g.segments * 32, g.segments * one, stream>>>(g);
+    LLME_LAUNCH_STATUS();
+}
+
 int sm_count() {
     static int n = [] {
         int dev = 0, v = 0;
@@ -293,6 +408,14 @@ int product(const float* A, const WT* W, float* C, int M, int N, int K, long lon
     g.vec_a = (uintptr_t)A % 16 == 0 && lda % 4 == 0 && sa % 4 == 0;
     g.vec_w = (uintptr_t)W % (4 * sizeof(WT)) == 0 && ldw % 4 == 0 && sw % 4 == 0;
     g.vec_c = (uintptr_t)C % 16 == 0 && ldc % 4 == 0 && sc % 4 == 0;
+    // Few rows stream the weights: 32 rows take 73 and 50 us against 119 and 74 in tiles, 48 rows (two passes) 115 and 95 against 121
+    // and 78.  (Copies of four values need the alignment; the tiles take everything.)
+    if (M <= FEW_ROWS && g.vec_a && g.vec_w) {
+        if (M <= 2) return launch_few<WT, 2>(g, batch, stream);
+        if (M <= 4) return launch_few<WT, 4>(g, batch, stream);
+        if (M <= 8) return launch_few<WT, 8>(g, batch, stream);
+        return M <= 16 ? launch_few<WT, 16>(g, batch, stream) : launch_few<WT, 32>(g, batch, stream);
+    }
     return dispatch(g, batch, stream);
 }
 

@@ -1,4 +1,4 @@
-"""The 32-bit product in each of its forms (tiles of 128, 64 and 16 rows, whole and shared by a cluster) at sizes around their edges:
+"""The 32-bit product in each of its forms (weights streamed for up to 2, 4, 8, 16 and 32 rows, tiles of 128, 64 and 16 rows, whole and shared by a cluster) at sizes around their edges:
 against 64 bits, and bit for bit the same row whatever else is in the launch."""
 import pytest
 import torch
@@ -9,14 +9,14 @@ DEV = "cuda:0"
 
 @pytest.mark.parametrize("N,K,w_dtype,pad", [
     (2048, 5504, torch.float32, 0), (1000, 1023, torch.float32, 0), (130, 2049, torch.bfloat16, 0), (64, 9001, torch.float32, 3), (11008, 2048, torch.float32, 0),
-    (300, 17, torch.bfloat16, 5), (4096, 16400, torch.bfloat16, 8)])
+    (300, 17, torch.bfloat16, 5), (4096, 16400, torch.bfloat16, 8), (50, 1030, torch.float32, 2), (4096, 16400, torch.float32, 4), (33, 6, torch.bfloat16, 2)])
 def test_every_form(N, K, w_dtype, pad):
     from llmengine_b200.kernels.ops import CudaOps
     ops, g = CudaOps(torch.device(DEV)), torch.Generator(device=DEV).manual_seed(N + K)
     x = torch.randn(601, K + pad, generator=g, device=DEV)[:, :K]
     w = torch.randn(N, K + pad, generator=g, device=DEV).to(w_dtype)[:, :K]
     outs = {}
-    for M in (1, 16, 17, 65, 129, 300, 601):
+    for M in (1, 2, 3, 5, 8, 9, 16, 17, 32, 33, 65, 129, 300, 601):
         out = torch.full((M, N + pad), 5.0, device=DEV)
         ops.linear(x[:M], w, out[:, :N])
         assert bool((out[:, N:] == 5.0).all())
