@@ -83,7 +83,8 @@ __device__ __forceinline__ bool wait_cluster(unsigned long long* bar, unsigned p
     atomicCAS(&g_status, 0, where);
     return false;
 }
-// arms a barrier (of either block) for bytes that TMA loads will bring; orders nothing that this thread has written
+// arms a barrier (of either block) for bytes that TMA loads will bring; orders nothing by itself: writes that the waiting block is to
+// see need a fence of cluster scope in front
 __device__ __forceinline__ void arrive_expect_cluster(unsigned cluster_addr, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr), "r"(bytes) : "memory");
 }
@@ -228,11 +229,15 @@ latent_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("fence.acq_rel.cluster;" ::: "memory");
             }
             __syncwarp();
             const unsigned full = map_to_cta(smem_u32(&bar->full[at_s]), 0);
-            if (lane == 0) arrive_expect_cluster(full, (unsigned)__popc(whole_mask) * (unsigned)(bs * 128));
+            if (lane == 0) {
+                // rows written by hand: the warp's writes, which this lane knows of from __syncwarp(), come before its arrival for
+                // the block that waits (a fence in front of __syncwarp() would order this lane's own only)
+                if (hand) asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                arrive_expect_cluster(full, (unsigned)__popc(whole_mask) * (unsigned)(bs * 128));
+            }
             __syncwarp();
             if (whole) tma_load_2d_pair(stage + cc * CHUNK + (box << bs_shift) * 128, &map_c, x0 + cc * 64, row, full);
         };
