@@ -913,16 +913,19 @@ LLME_API long long llme_attention_decode_scratch_floats(int n_rows, int nh, int 
     return splits <= 1 ? 0 : (long long)COUNTER_WORDS + (long long)n_rows * nh * splits * PART;
 }
 
+template <bool EXT>
+static LlmeGrants& decode_grants() {
+    static LlmeGrants grants;
+    return grants;
+}
+
 // How many clusters of `splits` blocks of the decode kernel the GPU holds at once (0: unknown).  A cluster's blocks
 // must find room in one GPC together, so this is less than the blocks the SMs hold divided by the cluster's size.
 LLME_API int llme_attention_decode_clusters(int splits) {
     if (splits < 2 || splits > 8) return 0;
     static int known[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     if (known[splits]) return known[splits];
-    if (cudaFuncSetAttribute(attention_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DECODE_SMEM) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
+    if (llme_grant_smem(decode_grants<false>(), attention_decode_kernel<false>, DECODE_SMEM) != cudaSuccess) return 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)splits, 1024, 1);
     cfg.blockDim = dim3(THREADS);
@@ -947,12 +950,9 @@ LLME_API int llme_attention_portion(const FastAttnArgs* args, int max_q_len, cud
     const FastAttnArgs& a = *args;
     if (a.n_rows <= 0 || max_q_len <= 0) return 0;
     if (int rc = check_common(a)) return rc;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_portion_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PORTION_SMEM);
-        if (e != cudaSuccess) LLME_REFUSE("attention: cannot reserve %zu bytes of shared memory: %s", PORTION_SMEM, cudaGetErrorString(e));
-        configured = true;
-    }
+    static LlmeGrants grants;
+    if (cudaError_t e = llme_grant_smem(grants, attention_portion_kernel, PORTION_SMEM))
+        LLME_REFUSE("attention: cannot reserve %zu bytes of shared memory: %s", PORTION_SMEM, cudaGetErrorString(e));
     const int G = a.nh / a.nkv;
     const long long tiles = ((long long)max_q_len * G + BM - 1) / BM;
     if (tiles > 2147483647LL || a.nkv > 65535) LLME_REFUSE("attention: grid too large");
@@ -967,12 +967,8 @@ static int launch_decode(const FastAttnArgs& a, const FusedQkv& f, const DecodeE
     if (int rc = check_common(a, f.qkv != nullptr)) return rc;
     if (a.splits < 1 || a.splits > 1024) LLME_REFUSE("attention: splits must be in 1..1024, got %d", a.splits);
     if (a.splits > 1 && !a.scratch) LLME_REFUSE("attention: split decoding needs scratch memory");
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel<EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DECODE_SMEM);
-        if (e != cudaSuccess) LLME_REFUSE("attention: cannot reserve %zu bytes of shared memory: %s", DECODE_SMEM, cudaGetErrorString(e));
-        configured = true;
-    }
+    if (cudaError_t e = llme_grant_smem(decode_grants<EXT>(), attention_decode_kernel<EXT>, DECODE_SMEM))
+        LLME_REFUSE("attention: cannot reserve %zu bytes of shared memory: %s", DECODE_SMEM, cudaGetErrorString(e));
     const int G = a.nh / a.nkv;
     const int chunks = (G + 15) / 16;
     if ((long long)a.nkv * chunks > 65535) LLME_REFUSE("attention: grid too large");

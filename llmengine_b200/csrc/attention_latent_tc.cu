@@ -446,14 +446,9 @@ size_t smem_bytes(int rot) {
 template <int RG, int BN>
 int launch(const Args& a, int n_list, int max_q_len, cudaStream_t stream) {
     const size_t smem = smem_bytes<RG, BN>(a.rot);
-    static size_t allowed = 0;
-    if (smem > allowed) {
-        if (cudaFuncSetAttribute(latent_attention_tc_kernel<RG, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            cudaGetLastError();
-            LLME_REFUSE("latent attention: rows of %d values need %zu bytes of shared memory", RANK + a.rot, smem);
-        }
-        allowed = smem;
-    }
+    static LlmeGrants grants;
+    if (llme_grant_smem(grants, latent_attention_tc_kernel<RG, BN>, smem) != cudaSuccess)
+        LLME_REFUSE("latent attention: rows of %d values need %zu bytes of shared memory", RANK + a.rot, smem);
     const int BM = 16 * RG;
     dim3 grid(((long long)max_q_len * a.nh + BM - 1) / BM, n_list, a.splits);
     llme_launch(latent_attention_tc_kernel<RG, BN>, grid, dim3(WARPS * 32), smem, stream, a);

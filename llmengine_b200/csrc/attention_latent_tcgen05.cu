@@ -518,12 +518,8 @@ LLME_API int llme_latent_pair(const LlmeFastAttnArgs* f, long long q_rows, long 
     Args a = {(const bf16*)f->cache, (bf16*)f->out, sink, f->rows, f->cu_q_lens, f->ctx_lens, f->table_rows, f->block_tables,
               f->max_blocks, f->nh, width, f->page_size, stages_for(chunks), f->scale, f->window};
     const size_t smem = smem_bytes(chunks, a.stages);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(latent_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-        if (e != cudaSuccess) LLME_REFUSE("latent attention: cannot reserve shared memory: %s", cudaGetErrorString(e));
-        configured = true;
-    }
+    static LlmeGrants grants;
+    if (cudaError_t e = llme_grant_smem(grants, latent_pair_kernel, smem)) LLME_REFUSE("latent attention: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     const long long pairs = ((long long)max_q_len * f->nh + PAIR_ROWS - 1) / PAIR_ROWS;
     if (pairs > (1 << 29)) LLME_REFUSE("latent attention: too many rows for one launch");
     latent_pair_kernel<<<dim3((unsigned)(2 * pairs), f->n_rows), BLOCK, smem, stream>>>(mq, mc, a);

@@ -325,12 +325,8 @@ LLME_API int llme_maps_decode(const LlmeMapsDecodeArgs* args, cudaStream_t strea
     if (((uintptr_t)a.q | (uintptr_t)a.cache) & 15) LLME_REFUSE("maps_decode: operands must be 16-byte aligned");
     const int units = a.groups * ((a.heads / a.groups + HEADS - 1) / HEADS);
     if (units > 65535 || a.n_rows > 65535) LLME_REFUSE("maps_decode: too many heads or requests for one launch");
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(maps_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
-            LLME_REFUSE("maps_decode: %d bytes of shared memory are not available", SMEM_BYTES);
-        configured = true;
-    }
+    static LlmeGrants grants;
+    if (llme_grant_smem(grants, maps_decode_kernel, SMEM_BYTES) != cudaSuccess) LLME_REFUSE("maps_decode: %d bytes of shared memory are not available", SMEM_BYTES);
     llme_launch(maps_decode_kernel, dim3(a.splits, units, a.n_rows), dim3(THREADS), (size_t)SMEM_BYTES, stream, a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

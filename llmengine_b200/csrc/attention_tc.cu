@@ -858,12 +858,9 @@ LLME_API int llme_attention_tc(const void* q, long long q_tokens, long long tota
     const bool ext = a.sink || (a.keep_first > 0 && a.window > 0) || a.softcap > 0.0f;
     if (ext && MAPS == 2) LLME_REFUSE("attention_tc: the form for two maps takes no sink, kept first positions or cap");
     auto kernel = ext ? attention_tc_kernel<MAPS == 1> : attention_tc_kernel<false>;
-    static bool configured[2] = {false, false};
-    if (!configured[ext]) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-        if (e != cudaSuccess) LLME_REFUSE("attention_tc: cannot reserve %zu bytes of shared memory: %s", SMEM_BYTES, cudaGetErrorString(e));
-        configured[ext] = true;
-    }
+    static LlmeGrants grants[2];
+    if (cudaError_t e = llme_grant_smem(grants[ext], kernel, SMEM_BYTES))
+        LLME_REFUSE("attention_tc: cannot reserve %zu bytes of shared memory: %s", SMEM_BYTES, cudaGetErrorString(e));
     const long long tiles = ((long long)max_q_len * G + BLOCK_ROWS - 1) / BLOCK_ROWS;
     if (tiles * (a.nkv / MAPS) > 2147483647LL) LLME_REFUSE("attention_tc: grid too large");
     dim3 grid((unsigned)(tiles * (a.nkv / MAPS)), 1, a.n_rows);

@@ -354,12 +354,8 @@ LLME_API int llme_window_attention_tc(const LlmeWindowFastArgs* args, int max_q_
     if (a.value_share > 1 && a.nkv % a.value_share) LLME_REFUSE("window attention: %d key heads do not share values %d at a time", a.nkv, a.value_share);
     if (a.nkv > 65535 || a.n_rows > 65535) LLME_REFUSE("window attention: more than 65535 key/value heads or requests");
     if ((((uintptr_t)a.q | (uintptr_t)a.cache | (uintptr_t)a.out) & 15)) LLME_REFUSE("window attention: operands must be 16-byte aligned");
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(window_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
-            LLME_REFUSE("window attention: %d bytes of shared memory are not available", SMEM_BYTES);
-        configured = true;
-    }
+    static LlmeGrants grants;
+    if (llme_grant_smem(grants, window_tc_kernel, SMEM_BYTES) != cudaSuccess) LLME_REFUSE("window attention: %d bytes of shared memory are not available", SMEM_BYTES);
     const int G = a.nh / a.nkv;
     const long long tiles = ((long long)max_q_len * G + BM - 1) / BM;
     if (a.splits > 1) {

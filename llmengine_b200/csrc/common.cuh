@@ -58,6 +58,32 @@ inline char* llme_error_buffer() {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// How much dynamic shared memory a kernel may take is an attribute of the kernel on ONE device.  A launcher keeps an LlmeGrants per
+// kernel (static) and asks for its bytes before every launch; the attribute is set the first time on each device, and again only when
+// a launch there needs more.
+#include <atomic>
+#include <mutex>
+struct LlmeGrants {
+    static constexpr int DEVICES = 64;              // (devices beyond these are asked every time)
+    std::atomic<size_t> bytes[DEVICES];
+    std::mutex change;
+};
+template <typename K>
+inline cudaError_t llme_grant_smem(LlmeGrants& grants, K* kernel, size_t bytes) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) {
+        std::atomic<size_t>* known = device < LlmeGrants::DEVICES ? &grants.bytes[device] : nullptr;
+        if (known && known->load(std::memory_order_acquire) >= bytes) return cudaSuccess;
+        std::lock_guard<std::mutex> one(grants.change);          // a smaller request of another thread must not follow a larger one
+        if (known && known->load(std::memory_order_relaxed) >= bytes) return cudaSuccess;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e == cudaSuccess && known) known->store(bytes, std::memory_order_release);
+    }
+    if (e != cudaSuccess) cudaGetLastError();       // (reported by the caller, not by the next launch)
+    return e;
+}
+
 #include <stdlib.h>
 #include <string.h>
 #include <utility>

@@ -477,12 +477,9 @@ template <int L, int M, int C, int W, int NS>
 int launch_tile(const LlmeDeltaArgs& a, int vec_state, cudaStream_t s) {
     using Tile = DeltaTile<L, M, C, W, NS>;
     auto kernel = delta_tile_kernel<L, M, C, W, NS>;
-    static bool configured = false;
-    if (!configured) {
-        if (sizeof(Tile) > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Tile)) != cudaSuccess)
-            LLME_REFUSE("delta_rule: %zu bytes of shared memory are not available", sizeof(Tile));
-        configured = true;
-    }
+    static LlmeGrants grants;
+    if (sizeof(Tile) > 48 * 1024 && llme_grant_smem(grants, kernel, sizeof(Tile)) != cudaSuccess)
+        LLME_REFUSE("delta_rule: %zu bytes of shared memory are not available", sizeof(Tile));
     // An ordinary launch, which waits for the kernel before it: let in early, the blocks would crowd on the first SMs that have
     // room (there are about as many blocks as SMs), and the walk would take twice its time.
     kernel<<<dim3((a.p + Tile::COLS - 1) / Tile::COLS, a.heads, a.n_rows), 32 * W, sizeof(Tile), s>>>(a, vec_state);

@@ -221,12 +221,8 @@ int launch(const Problem<WT>& g, int batch, cudaStream_t stream) {
     constexpr int BM = 16 * TM, BN = 16 * TN;
     constexpr size_t stages = sizeof(Tile<TM, TN>), part = SPLIT ? (size_t)BM * BN * 4 : 0, smem = stages > part ? stages : part;
     auto kernel = gemm_nt_f32_kernel<WT, TM, TN, SPLIT>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) LLME_REFUSE("gemm_f32: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-        configured = true;
-    }
+    static LlmeGrants grants;
+    if (cudaError_t e = llme_grant_smem(grants, kernel, smem)) LLME_REFUSE("gemm_f32: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, SPLIT ? batch * g.segments : batch);
     cfg.blockDim = dim3(THREADS);
@@ -348,12 +344,9 @@ template <typename WT, int MT>
 int launch_few(const Problem<WT>& g, int batch, cudaStream_t stream) {
     constexpr int one = few_stages(MT) * few_stage_bytes<WT, MT>();
     auto kernel = gemm_few_f32_kernel<WT, MT>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SEGMENTS * one);
-        if (e != cudaSuccess) LLME_REFUSE("gemm_f32: cannot reserve %d bytes of shared memory: %s", MAX_SEGMENTS * one, cudaGetErrorString(e));
-        configured = true;
-    }
+    static LlmeGrants grants;
+    if (cudaError_t e = llme_grant_smem(grants, kernel, MAX_SEGMENTS * one))
+        LLME_REFUSE("gemm_f32: cannot reserve %d bytes of shared memory: %s", MAX_SEGMENTS * one, cudaGetErrorString(e));
     kernel<<<dim3((g.N + FEW_N - 1) / FEW_N, (g.M + MT - 1) / MT, batch), g.segments * 32, g.segments * one, stream>>>(g);
     LLME_LAUNCH_STATUS();
 }

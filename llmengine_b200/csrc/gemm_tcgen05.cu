@@ -328,12 +328,8 @@ int launch_kernel(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMa
     constexpr size_t smem = 1024 + (size_t)STAGES * (BM + (PAIR ? BN / 2 : BN)) * BK * 2 + (TMA_STORE ? 4 * 2 * 4096 : 0) + (2 * STAGES + 4) * 8 + 16;
     static_assert(smem <= 232448, "the block's shared memory must fit an SM");
     auto kernel = PAIR ? gemm_tc_pair_kernel<BN, STAGES, O, TMA_STORE, ACT> : gemm_tc_kernel<BN, STAGES, O, TMA_STORE, ACT>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) LLME_REFUSE("gemm_tc: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-        configured = true;
-    }
+    static LlmeGrants grants;
+    if (cudaError_t e = llme_grant_smem(grants, kernel, smem)) LLME_REFUSE("gemm_tc: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     const int tiles = a.m_tiles * a.n_tiles;
     int walkers = PAIR ? sm_count() / 2 : sm_count();                     // blocks, or pairs of blocks
     if (PAIR) {

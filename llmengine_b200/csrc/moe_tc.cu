@@ -329,14 +329,8 @@ int launch(const LlmeGroupedArgs& a, cudaStream_t s) {
         return -1;
     }
     auto kernel = grouped_tc_kernel<BM, BN, WM, WNW, STAGES, ACT, O>;
-    static bool configured = false;
-    if (!configured) {
-        if (SMEM > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) {
-            snprintf(llme_error_buffer(), 512, "grouped_linear_tc: %d bytes of shared memory are not available", SMEM);
-            return -1;
-        }
-        configured = true;
-    }
+    static LlmeGrants grants;
+    if (SMEM > 48 * 1024 && llme_grant_smem(grants, kernel, SMEM) != cudaSuccess) LLME_REFUSE("grouped_linear_tc: %d bytes of shared memory are not available", SMEM);
     llme_launch(kernel, dim3((n_out + BN - 1) / BN, tiles), dim3(32 * WM * WNW), (size_t)SMEM, s, a);
     LLME_LAUNCH_STATUS();
 }

@@ -259,12 +259,8 @@ int launch(const LlmeGroupedArgs& a, const void* x, long long ldx, cudaStream_t 
     if (int rc = make_map(&mx, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.pairs, a.k, ldx, BM, BK)) return rc;
     if (int rc = make_map(&mw, a.w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (long long)a.num_experts * a.n, a.k, a.ldw, BN / 2, BK)) return rc;
     auto kernel = grouped_tcgen05_kernel<ACT, O>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
-        if (e != cudaSuccess) LLME_REFUSE("grouped_tcgen05: cannot reserve %zu bytes of shared memory: %s", SMEM, cudaGetErrorString(e));
-        configured = true;
-    }
+    static LlmeGrants grants;
+    if (cudaError_t e = llme_grant_smem(grants, kernel, SMEM)) LLME_REFUSE("grouped_tcgen05: cannot reserve %zu bytes of shared memory: %s", SMEM, cudaGetErrorString(e));
     kernel<<<sm_count(), THREADS, SMEM, s>>>(mx, mw, a);
     LLME_LAUNCH_STATUS();
 }
