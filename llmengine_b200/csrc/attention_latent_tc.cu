@@ -457,12 +457,8 @@ int launch(const Args& a, int n_list, int max_q_len, cudaStream_t stream) {
 
 }  // namespace
 
-// 0 if no bounded wait ever gave up (synchronises the device).
-LLME_API int llme_latent_attention_tc_status() {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_status, sizeof(int)) != cudaSuccess) return -1;
-    return v;
-}
+// 0 if no bounded wait has given up since the last call (synchronises the device).
+LLME_API int llme_latent_attention_tc_status() { LLME_TAKE_STATUS(g_status); }
 
 // Whether rows of RANK + rot values fit the kernel (shared memory of the wider configuration).
 LLME_API int llme_latent_attention_tc_fits(int rot) {

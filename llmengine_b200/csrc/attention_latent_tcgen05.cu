@@ -494,13 +494,8 @@ LLME_API int llme_latent_pair_supports(int rot, int page_size) {
     return page_size == 8 || page_size == 16 || page_size == 32 || (page_size > 0 && page_size % 64 == 0);
 }
 
-// 0 if no bounded wait ever gave up (synchronises the device).
-LLME_API int llme_latent_pair_status() {
-    int v = 0;
-    cudaDeviceSynchronize();
-    cudaMemcpyFromSymbol(&v, g_status, sizeof v);
-    return v;
-}
+// 0 if no bounded wait has given up since the last call (synchronises the device).
+LLME_API int llme_latent_pair_status() { LLME_TAKE_STATUS(g_status); }
 
 // Requests `rows` of the step, each with any number of new tokens up to `max_q_len`; q has q_rows rows of RANK + rot values in all, the cache
 // cache_rows.

@@ -868,9 +868,5 @@ LLME_API int llme_attention_tc(const void* q, long long q_tokens, long long tota
     LLME_LAUNCH_STATUS();
 }
 
-LLME_API int llme_attention_tc_status() {
-    int v = 0, zero = 0;
-    if (cudaMemcpyFromSymbol(&v, g_status, sizeof(int)) != cudaSuccess) return -1;
-    if (v != 0) cudaMemcpyToSymbol(g_status, &zero, sizeof(int));
-    return v;
-}
+// 0 if no bounded wait has given up since the last call (synchronises the device).
+LLME_API int llme_attention_tc_status() { LLME_TAKE_STATUS(g_status); }

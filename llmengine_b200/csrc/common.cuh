@@ -39,6 +39,18 @@ inline char* llme_error_buffer() {
         return (int)e__;                                              \
     } while (0)
 
+// What the body of a library's ..._status() is: the flag in which its kernels record that a bounded wait gave up (0: none did; -1: it
+// could not be read), read when everything launched so far on the device has ended, and cleared, so that the next call speaks of what
+// came after this one.  `flag` is the library's __device__ int.
+#define LLME_TAKE_STATUS(flag)                                                                              \
+    do {                                                                                                    \
+        int v__ = 0;                                                                                        \
+        const int zero__ = 0;                                                                               \
+        if (cudaDeviceSynchronize() != cudaSuccess || cudaMemcpyFromSymbol(&v__, flag, sizeof(int)) != cudaSuccess) return -1; \
+        if (v__ != 0 && cudaMemcpyToSymbol(flag, &zero__, sizeof(int)) != cudaSuccess) return -1;           \
+        return v__;                                                                                         \
+    } while (0)
+
 // Programmatic dependent launch.  A kernel launched through llme_launch may begin while the kernel
 // before it in the stream is still running (its blocks become resident once every block of the earlier
 // kernel has started); what it reads from or writes to memory that the earlier kernel touches must come

@@ -471,10 +471,5 @@ LLME_API int llme_gemm_tc_gated_bf16(const void* x, long long ldx, const void* w
     return launch_act<256, 4, bf16, false>(x, ldx, w, ldw, a, stream);
 }
 
-// Reads and clears the error flag of the kernels (synchronises the device).  0 = no wait ever gave up.
-LLME_API int llme_gemm_tc_status() {
-    int v = 0, zero = 0;
-    if (cudaMemcpyFromSymbol(&v, g_status, sizeof(int)) != cudaSuccess) return -1;
-    if (v != 0) cudaMemcpyToSymbol(g_status, &zero, sizeof(int));
-    return v;
-}
+// 0 if no bounded wait has given up since the last call (synchronises the device).
+LLME_API int llme_gemm_tc_status() { LLME_TAKE_STATUS(g_status); }

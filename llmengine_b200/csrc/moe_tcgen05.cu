@@ -298,10 +298,5 @@ LLME_API int llme_grouped_tcgen05(const LlmeGroupedArgs* args, void* rows, int o
     return a.act == 1 ? launch<1, bf16>(a, x, ldx, stream) : a.act == 2 ? launch<2, bf16>(a, x, ldx, stream) : a.act == 3 ? launch<3, bf16>(a, x, ldx, stream) : launch<0, bf16>(a, x, ldx, stream);
 }
 
-// Reads and clears the error flag of the kernel (synchronises the device).  0 = no wait ever gave up.
-LLME_API int llme_grouped_tcgen05_status() {
-    int v = 0, zero = 0;
-    if (cudaMemcpyFromSymbol(&v, g_status, sizeof(int)) != cudaSuccess) return -1;
-    if (v != 0) cudaMemcpyToSymbol(g_status, &zero, sizeof(int));
-    return v;
-}
+// 0 if no bounded wait has given up since the last call (synchronises the device).
+LLME_API int llme_grouped_tcgen05_status() { LLME_TAKE_STATUS(g_status); }

@@ -425,17 +425,17 @@ class Engine:
     def free(self, request: Hashable) -> None:
         self.cache.free_request(request)
 
+    # libraries whose kernels wait with a limit -> what says whether a wait gave up (and forgets it)
+    _STATUS = {"gemm_tcgen05": "llme_gemm_tc_status", "moe_tcgen05": "llme_grouped_tcgen05_status", "attention_tc": "llme_attention_tc_status",
+               "attention_latent_tc": "llme_latent_attention_tc_status", "attention_latent_tcgen05": "llme_latent_pair_status"}
+
     def check_kernels(self) -> None:
-        """Raise if a bounded wait inside a kernel ever gave up (synchronises the device)."""
-        libs = getattr(self.ops, "_libs", {})
-        status = self.ops.linear_tc_status() if "gemm_tcgen05" in libs else 0
-        status = status or (self.ops.grouped_tcgen05_status() if "moe_tcgen05" in libs else 0)
-        for key in libs:
-            if key.startswith("attention_tc@HEAD_DIM="):
-                status = status or int(libs[key].llme_attention_tc_status())
-            if key.startswith("attention_latent_tc@"):
-                status = status or int(libs[key].llme_latent_attention_tc_status())
-            if key.startswith("attention_latent_tcgen05@"):
-                status = status or int(libs[key].llme_latent_pair_status())
-        if status:
-            raise RuntimeError(f"a tcgen05 kernel gave up waiting (code {status}): its results are not valid")
+        """Raise if a bounded wait inside a kernel has given up since the last call (synchronises the device)."""
+        gave_up = []
+        for key, lib in getattr(self.ops, "_libs", {}).items():
+            name = self._STATUS.get(key.partition("@")[0])
+            status = int(getattr(lib, name)()) if name else 0        # (of every library: a flag left unread would speak up in a later call)
+            if status:
+                gave_up.append(f"{key} (code {status})")
+        if gave_up:
+            raise RuntimeError(f"a wait inside a kernel gave up, the results are not valid: {', '.join(gave_up)}")

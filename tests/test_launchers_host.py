@@ -1,4 +1,5 @@
-"""Launchers against a stand-in for the CUDA runtime (`fake_cuda_runtime.cpp`): several devices in one process."""
+"""Launchers against a stand-in for the CUDA runtime (`fake_cuda_runtime.cpp`): several devices in one process, and the flags that tell
+of a wait that gave up."""
 import ctypes
 import os
 import subprocess
@@ -56,3 +57,40 @@ def test_latent_attention_on_a_second_device(compiled):
             for q_len in (1, 2, 100):
                 assert tc.llme_latent_attention_tc(ctypes.byref(args), None, c_int(rot), c_int(q_len), None) == 0
             assert pair.llme_latent_pair(ctypes.byref(args), c_longlong(1600), c_longlong(640), None, c_int(rot), c_int(100), None) == 0
+
+
+STATUS = {"gemm_tcgen05": "llme_gemm_tc_status", "moe_tcgen05": "llme_grouped_tcgen05_status", "attention_tc@HEAD_DIM=64": "llme_attention_tc_status",
+          "attention_latent_tc@RANK=128": "llme_latent_attention_tc_status", "attention_latent_tcgen05@RANK=128": "llme_latent_pair_status"}
+
+
+@pytest.mark.parametrize("key", sorted(STATUS))
+def test_a_status_is_told_once(compiled, key):
+    lib = compiled(key)
+    status = getattr(lib, STATUS[key])
+    assert status() == 0
+    lib.fake_flag(21, 0, 0)
+    assert status() == 21 and status() == 0                # told, and forgotten
+    lib.fake_flag(0, 7, 0)                                 # by a kernel that still runs: the device is waited for
+    assert status() == 7 and status() == 0
+    lib.fake_flag(0, 0, 1)                                 # a flag that cannot be read is not "fine"
+    assert status() == -1
+    lib.fake_flag(0, 0, 0)
+
+
+def test_every_flag_is_read_when_one_is_set():
+    """The engine reads (and thereby clears) all of them, names what gave up, and says nothing the next time."""
+    from types import SimpleNamespace
+
+    from llmengine_b200.engine.engine import Engine
+    flags = {"gemm_tcgen05": 0, "attention_latent_tc@RANK=64": 1, "attention_latent_tcgen05@RANK=512": 22, "elementwise": 0}
+
+    def lib(key):
+        def take():
+            v, flags[key] = flags[key], 0
+            return v
+        return SimpleNamespace(**{name: take for name in STATUS.values()})
+    eng = SimpleNamespace(ops=SimpleNamespace(_libs={k: lib(k) for k in flags}, linear_tc_status=lambda: 0), _STATUS=getattr(Engine, "_STATUS", None))
+    with pytest.raises(RuntimeError) as e:
+        Engine.check_kernels(eng)
+    assert "attention_latent_tc@RANK=64" in str(e.value) and "attention_latent_tcgen05@RANK=512" in str(e.value)
+    Engine.check_kernels(eng)
