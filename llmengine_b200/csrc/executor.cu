@@ -488,10 +488,14 @@ void fill_fast(LlmeFastAttnArgs& a, const LlmeAttendOp& o, const LlmeStep& s, co
     a.splits = splits; a.scale = o.scale;
 }
 
+long long attention_scratch_needed(LlmeExecutor& ex, int n_rows, int nh, int hd, int splits) {
+    auto* need = (AttnScratchFn)ex.find_hd("attention_decode_scratch", hd);
+    return need ? need(n_rows, nh, splits) : 65536 + (long long)n_rows * nh * splits * (hd + 2);
+}
+
 int scratch_check(LlmeExecutor& ex, const LlmeAttendOp& o, int n_rows, int splits) {
     if (splits <= 1) return 0;
-    auto* need = (AttnScratchFn)ex.find_hd("attention_decode_scratch", o.hd);
-    const long long floats = need ? need(n_rows, o.nh, splits) : 65536 + (long long)n_rows * o.nh * splits * (o.hd + 2);
+    const long long floats = attention_scratch_needed(ex, n_rows, o.nh, o.hd, splits);
     if (!o.scratch || floats > o.scratch_floats)
         return ex.fail("attention: %d requests x %d splits need %lld scratch values, the record has %lld", n_rows, splits, floats, o.scratch_floats);
     return 0;
@@ -836,8 +840,8 @@ int window_attend(LlmeExecutor& ex, const LlmeWindowAttentionOp& o, const LlmeSt
             aligned16(o.q, o.cache, o.out)) {
             LlmeAttendOp at = {o.q, o.out, o.dtype, o.cache, o.cache_pages * 2 * o.nkv * ps, o.group, o.nh, o.nkv, o.dk, o.window, o.scale,
                                o.decode_scratch, o.decode_scratch_floats};
-            const int splits = decode_splits(ex, s.num_decode, o.nh, o.nkv, o.dk, o.window, s.max_decode_ctx);
-            if (int rc = scratch_check(ex, at, s.num_decode, splits)) return rc;
+            int splits = decode_splits(ex, s.num_decode, o.nh, o.nkv, o.dk, o.window, s.max_decode_ctx);
+            while (splits > 1 && attention_scratch_needed(ex, s.num_decode, o.nh, o.dk, splits) > o.decode_scratch_floats) --splits;
             LlmeFastAttnArgs d = {};
             fill_fast(d, at, s, s.decode_rows, s.num_decode, splits);
             if (int rc = ex.launched(ext(&d, o.sink, o.keep_first, o.softcap, st), "attention_decode_ext")) return rc;

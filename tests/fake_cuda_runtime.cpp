@@ -44,6 +44,8 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { return *v = 14
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute, int bytes) { return granted[{device, f}] = bytes, cudaSuccess; }
 cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t smem, cudaStream_t) { return launch(f, smem); }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) { return launch(f, c->dynamicSmemBytes); }
+cudaError_t cudaMalloc(void** p, size_t) { return *p = nullptr, cudaErrorMemoryAllocation; }
+cudaError_t cudaFree(void*) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { cudaError_t e = last; return last = cudaSuccess, e; }
 const char* cudaGetErrorString(cudaError_t) { return "refused by the stand-in"; }
 cudaError_t cudaDeviceSynchronize() {

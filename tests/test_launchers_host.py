@@ -1,5 +1,5 @@
 """Launchers against a stand-in for the CUDA runtime (`fake_cuda_runtime.cpp`): several devices in one process, and the flags that tell
-of a wait that gave up."""
+of a wait that gave up; and what the step executor hands to the kernels that it chooses."""
 import ctypes
 import os
 import subprocess
@@ -22,7 +22,7 @@ def compiled(tmp_path_factory):
             name, defines = build.split_key(key)
             at = os.path.join(str(folder), f"lib{len(done)}.so")
             subprocess.run([build.find_nvcc(), "-gencode", "arch=compute_100a,code=compute_100a", "-std=c++17", "-O1", "--shared", "-cudart", "none", "-Xcompiler", "-fPIC",
-                            "-Xlinker", "-Bsymbolic", *defines, os.path.join(build.CSRC, build.SOURCES[name]), os.path.join(HERE, "fake_cuda_runtime.cpp"), "-o", at], check=True)
+                            "-Xlinker", "-Bsymbolic", *defines, os.path.join(build.CSRC, build.SOURCES[name]), os.path.join(HERE, "fake_cuda_runtime.cpp"), "-I", build.INCLUDE, *build.LINK.get(name, []), "-o", at], check=True)
             done[key] = ctypes.CDLL(at)
         return done[key]
     return get
@@ -94,3 +94,60 @@ def test_every_flag_is_read_when_one_is_set():
         Engine.check_kernels(eng)
     assert "attention_latent_tc@RANK=64" in str(e.value) and "attention_latent_tcgen05@RANK=512" in str(e.value)
     Engine.check_kernels(eng)
+
+
+class _Executor:
+    """The step executor with stand-ins for its kernels, which keep what they were given."""
+
+    def __init__(self, lib):
+        from llmengine_b200.kernels import executor as ex
+        self.lib, self.ex, self.given, self._keep = lib, ex, {}, []
+        lib.llme_executor_create.restype = lib.llme_plan_create.restype = c_void_p
+        lib.llme_executor_error.restype = ctypes.c_char_p
+        self.handle = c_void_p(lib.llme_executor_create(0))
+
+    def kernel(self, name, *types, takes=0, result=0, restype=c_int):
+        """Registers a kernel of these argument types; argument `takes`, a structure's address, is kept under its name."""
+        def called(*args):
+            self.given[name] = args[takes].contents if hasattr(args[takes], "contents") else args
+            return result(*args) if callable(result) else result
+        fn = ctypes.CFUNCTYPE(restype, *types)(called)
+        self._keep.append(fn)
+        assert self.lib.llme_executor_register(self.handle, name.encode(), ctypes.cast(fn, c_void_p)) == 0
+
+    def run(self, kind, record, step):
+        plan = c_void_p(self.lib.llme_plan_create(self.handle))
+        assert self.lib.llme_plan_add(plan, c_int(kind), ctypes.byref(record), ctypes.c_size_t(ctypes.sizeof(record))) == 0
+        rc = self.lib.llme_plan_run(plan, ctypes.byref(step), c_int(0), c_int(1), None)
+        assert rc == 0, self.lib.llme_executor_error(self.handle)
+
+
+def _window_step(compiled, requests, heads, kv_heads, window, keep_first, ctx, scratch_floats):
+    """The argument block of the split-context kernel for `requests` single tokens with a sink."""
+    from ctypes import POINTER
+    e = _Executor(compiled("executor"))
+    P, far = c_void_p, 1 << 24
+    e.kernel("window_post", P, c_int, P)
+    e.kernel("window_attention_tc/128x128", P, c_int, c_int, P)
+    e.kernel("attention_decode/128", P, P)
+    e.kernel("attention_portion/128", P, c_int, P)
+    e.kernel("attention_decode_scratch/128", c_int, c_int, c_int, result=lambda n, h, s: 0 if s <= 1 else 65536 + n * h * s * 130, restype=c_longlong)
+    e.kernel("attention_decode_ext/128", POINTER(_Fast), P, c_int, c_float, P)
+    op = e.ex.WindowAttentionOp()
+    op.q_in = op.k_in = op.v_in = op.q = op.out = op.cache = op.sink = op.decode_scratch = far
+    op.dtype, op.nh, op.nkv, op.dk, op.dv, op.window, op.keep_first, op.scale, op.amplitude = 1, heads, kv_heads, 128, 128, window, keep_first, 0.1, 1.0
+    op.decode_scratch_floats, op.cache_pages, op.value_share = scratch_floats, 4096, 1
+    step = e.ex.Step()
+    step.num_tokens = step.num_requests = step.num_decode = requests
+    step.max_decode_ctx, step.num_groups = ctx, 1
+    step.groups[0] = e.ex.StepGroup(far, far, 1024, 16, window)
+    e.run(e.ex.OP_WINDOW_ATTENTION, op, step)
+    return e.given["attention_decode_ext/128"]
+
+
+def test_shares_are_fewer_where_the_scratch_memory_is_small(compiled):
+    """Any scratch memory is enough for one share; more shares only as far as their partial results fit."""
+    most = _window_step(compiled, 2, 16, 4, 0, 0, 8000, 1 << 30).splits
+    assert most > 3
+    assert _window_step(compiled, 2, 16, 4, 0, 0, 8000, 1).splits == 1
+    assert _window_step(compiled, 2, 16, 4, 0, 0, 8000, 65536 + 2 * 16 * 3 * 130).splits == 3
