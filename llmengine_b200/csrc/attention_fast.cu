@@ -581,20 +581,33 @@ __global__ void __launch_bounds__(THREADS) attention_decode_kernel(FastAttnArgs 
     // global memory one by one, in front of every sub-tile's copies, each entry cost a warp a memory
     // round trip (8 of them per warp at 2,048 cached tokens, about a third of the kernel's time).
     __shared__ int page_tab[PAGE_TAB];
-    const int* tab = bt;
-    int tab_first = 0;
-    if (my_first <= my_last && my_last >= sub_first) {
-        const int start = max(my_first, sub_first) * SUB, blk_first = (EXT && kept > start ? start : max(start, lo)) / ps, blk_last = min(my_last * SUB + SUB - 1, p) / ps;
-        if (blk_last - blk_first < PAGE_TAB) {
-            for (int i = threadIdx.x; i <= blk_last - blk_first; i += THREADS) page_tab[i] = bt[blk_first + i];
-            tab = page_tab;
-            tab_first = blk_first;
-            __syncthreads();
+    const int *tab = bt, *front_tab = bt;
+    int tab_first = 0, front_first = 0;
+    if (my_first <= my_last) {
+        int held = 0;
+        if (my_last >= sub_first) {
+            const int start = max(my_first, sub_first) * SUB, blk_first = (EXT && kept > start ? start : max(start, lo)) / ps, blk_last = min(my_last * SUB + SUB - 1, p) / ps;
+            if (blk_last - blk_first < PAGE_TAB) {
+                for (int i = threadIdx.x; i <= blk_last - blk_first; i += THREADS) page_tab[i] = bt[blk_first + i];
+                tab = page_tab;
+                tab_first = blk_first;
+                held = blk_last - blk_first + 1;
+            }
         }
+        if (EXT && my_first < sub_first) {                           // behind them the kept first positions' part
+            const int blk_first = first_key(my_first) / ps, n = (min(first_key(min(my_last, sub_first - 1)) + SUB, kept) - 1) / ps - blk_first + 1;
+            if (held + n <= PAGE_TAB) {
+                for (int i = threadIdx.x; i < n; i += THREADS) page_tab[held + i] = bt[blk_first + i];
+                front_tab = page_tab + held;
+                front_first = blk_first;
+                held += n;
+            }
+        }
+        if (held) __syncthreads();
     }
     auto load_sub = [&](bf16* dst, int sub) {
-        const bool front = EXT && sub < sub_first;                   // (in front of the part of the table that was copied)
-        load_sub_tile(dst, a.cache, front ? bt : tab, front ? 0 : tab_first, kvh, a.nkv, ps, page_shift, first_key(sub), lo, p, kept);
+        const bool front = EXT && sub < sub_first;
+        load_sub_tile(dst, a.cache, front ? front_tab : tab, front ? front_first : tab_first, kvh, a.nkv, ps, page_shift, first_key(sub), lo, p, kept);
     };
     const float* cs_row = nullptr;
     if (f.qkv && f.cos_sin) {

@@ -840,7 +840,9 @@ int window_attend(LlmeExecutor& ex, const LlmeWindowAttentionOp& o, const LlmeSt
             aligned16(o.q, o.cache, o.out)) {
             LlmeAttendOp at = {o.q, o.out, o.dtype, o.cache, o.cache_pages * 2 * o.nkv * ps, o.group, o.nh, o.nkv, o.dk, o.window, o.scale,
                                o.decode_scratch, o.decode_scratch_floats};
-            int splits = decode_splits(ex, s.num_decode, o.nh, o.nkv, o.dk, o.window, s.max_decode_ctx);
+            // the keys that a token sees: its window's and the kept first ones
+            const long long seen = (long long)o.window + o.keep_first;
+            int splits = decode_splits(ex, s.num_decode, o.nh, o.nkv, o.dk, o.window > 0 && seen < s.max_decode_ctx ? (int)seen : 0, s.max_decode_ctx);
             while (splits > 1 && attention_scratch_needed(ex, s.num_decode, o.nh, o.dk, splits) > o.decode_scratch_floats) --splits;
             LlmeFastAttnArgs d = {};
             fill_fast(d, at, s, s.decode_rows, s.num_decode, splits);

@@ -145,6 +145,14 @@ def _window_step(compiled, requests, heads, kv_heads, window, keep_first, ctx, s
     return e.given["attention_decode_ext/128"]
 
 
+def test_kept_first_positions_count_as_keys(compiled):
+    """A token sees its window and the kept first positions: as many shares as a window of all of them would get."""
+    for requests in (1, 2, 5):
+        kept = _window_step(compiled, requests, 16, 4, 128, 4096, 8000, 1 << 30).splits
+        assert kept == _window_step(compiled, requests, 16, 4, 4224, 0, 8000, 1 << 30).splits > 3
+        assert _window_step(compiled, requests, 16, 4, 128, 1 << 30, 8000, 1 << 30).splits >= kept      # never more keys than there are
+
+
 def test_shares_are_fewer_where_the_scratch_memory_is_small(compiled):
     """Any scratch memory is enough for one share; more shares only as far as their partial results fit."""
     most = _window_step(compiled, 2, 16, 4, 0, 0, 8000, 1 << 30).splits
