@@ -12,7 +12,7 @@
 //
 //   warps 0..3  softmax: a thread owns half of a row's keys (lanes 0..63: the tile's first 64, lanes 64..127: the others), the two
 //               threads of a row tell each other their maxima; P goes to shared memory (the A operand of O += P V).  The outputs
-//               are rescaled only when a row's maximum has grown by more than 2^8.
+//               are rescaled only when a row's maximum has grown by more than 2^8 or its weight asks for it.
 //   warp 4      of the first block issues the pair's instructions: S(0) S(1) | O(0) S(2) | O(1) S(3) | ...
 //   warps 5..8  TMA, page by page through the block table, 64 columns x 64 keys at a time, into a ring of 16 KB stages, in turn; the
 //               barrier of a stage lives in the first block and counts both blocks' bytes.  The keys run two tiles ahead of the
@@ -66,6 +66,7 @@ struct Barriers {
     unsigned tmem_base;
     int abort_flag;
     float row_max[2][2][ROWS];     // [tile parity][half of the keys][row]
+    float row_l[2][2][ROWS];       // likewise: the sums before the tile
     float row_sum[2][ROWS];
 };
 
@@ -349,6 +350,7 @@ latent_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         const bool with_sink = a.sink != nullptr && row_ok;
         float m_ref = with_sink ? a.sink[g_row % H] * LOG2E : -INFINITY;
         float l_run = with_sink && kh == 0 ? 1.0f : 0.0f;       // the sink counts once
+        bool unseen = true;                                     // no key of the row so far
         bool ok = true;
         for (int i = 0; i < n_tiles; ++i) {
             const int b = i & 1, j0 = (tile_first + i) * BN + kh * 64;
@@ -375,10 +377,16 @@ latent_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             }
             // (both threads of a row come here once per tile, also after a wait has given up)
             bar->row_max[b][kh][row] = own;
+            bar->row_l[b][kh][row] = l_run;
             pair_sync();
             if (!ok) continue;
             const float m_true = fmaxf(own, bar->row_max[b][kh ^ 1][row]) * sc;
-            const bool move = m_true > m_ref + RESCALE || (m_ref == -INFINITY && m_true > -INFINITY);
+            // Relative to the row's true maximum the largest probability is one, which bfloat16 holds exactly; relative to an older
+            // reference, or to the sink, it is rounded like the others.  It is kept exact where it weighs: in the first tile that the
+            // row sees, and where it is more than a 64th of the row's sum.  Error of the layer, a 2,000-token prompt (the warp-level
+            // kernel: 4.2194e-3): 4.2285e-3 with neither this nor the rounded probabilities' sum, 4.2215e-3 with the latter, 4.2183e-3 with both.
+            const bool move = m_true > m_ref + RESCALE || (m_true > m_ref && (unseen || fast_exp2(m_true - m_ref) * 64.0f > l_run + bar->row_l[b][kh ^ 1][row]));
+            unseen = unseen && m_true == -INFINITY;
             if (__any_sync(0xffffffffu, move)) {
                 const float m_new = move ? m_true : m_ref;
                 const float corr = move ? fast_exp2(m_ref - m_new) : 1.0f;      // (exp2 of -inf: 0, nothing had been seen)
@@ -415,8 +423,10 @@ latent_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     const int at = q * 8 + 2 * e;
                     const float e0 = fast_exp2(fmaf(__uint_as_float(v[at >> 5][at & 31]), sc, -ref));          // a masked score is -inf: exactly 0
                     const float e1 = fast_exp2(fmaf(__uint_as_float(v[at >> 5][(at & 31) + 1]), sc, -ref));
-                    sum[e] += e0 + e1;
-                    pw[e] = pack2(e0, e1);
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(e0, e1);
+                    const float2 rounded = __bfloat1622float2(h);        // the sum of what is multiplied with the values
+                    sum[e] += rounded.x + rounded.y;
+                    pw[e] = *reinterpret_cast<const unsigned*>(&h);
                 }
                 *reinterpret_cast<uint4*>(p_row + ((q ^ (row & 7)) << 4)) = pk;
             }
