@@ -14,6 +14,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
+#include <cmath>
 #include <map>
 #include <string>
 #include <vector>
@@ -999,17 +1001,31 @@ int op_moe_route(LlmeExecutor& ex, const LlmeMoeRouteOp& o, const LlmeStep& s, c
 // this kernel against the warp-level ones: 16 tokens (2 rows) 153 / 143 us, 32 (4 rows) 175 / 186, 96 177 / 220, 250 185 / 446, 500 198 / 395.
 constexpr long long GROUPED_ROWS = 4;
 
+// Below that: the weight-streaming form or the tcgen05 kernel, whichever these estimates of their times (us) give less.  A streaming block
+// serves 16 weight rows of an expert and two are on an SM at a time; it takes 2.6 us however few values of k it reads, k / 610 where those
+// are many, and longer to find its expert among many; blocks beyond the routing's own tiles cost that search.  The tcgen05 kernel
+// takes some 12 us to start and drain (with the gather in front 19), a tile of 128 weight rows an SM k / 170.  Experts that have rows
+// are counted for an even routing.  Measured over eleven pairs of products (8 to 128 experts of 1,024 to 4,096 rows, k = 512 to 2,048, a
+// quarter to four rows an expert, even and skewed routing): never more than 4 % above the better of the two.  128 experts,
+// 2048 x 512, 24 tokens of 8 choices: 123 us streaming, 39 tcgen05 (59 the 16-row tiles of before); 32 experts, 4096 x 2048, 8 tokens of 4: 61 and 74 (114).
+bool grouped_streams(const LlmeExecutor& ex, const LlmeGroupedArgs& a) {
+    const double E = a.num_experts, pairs = a.pairs, used = E * (1.0 - std::exp(-pairs / E));
+    const double launched = std::min(pairs, std::floor((pairs + 7.0) / 8.0) + std::min(E, pairs));
+    const double stream = 2.5 + a.n / 16.0 * (used * (std::max(2.6, a.k / 610.0) + 0.0025 * E) + std::max(0.0, launched - used) * 0.0075 * E) / (2.0 * ex.sms);
+    const double tiles = 12.0 + (a.gather ? 6.7 : 0.0) + std::max(1.0, used * a.n / 128.0 / ex.sms) * a.k / 170.0;
+    return stream <= tiles;
+}
+
 int op_grouped_linear(LlmeExecutor& ex, const LlmeGroupedLinearOp& o, const LlmeStep& s, cudaStream_t st) {
     if (s.num_tokens <= 0) return 0;
     LlmeGroupedArgs a = {o.x, o.ldx, o.w, o.ldw, o.w_expert, o.out, o.ldo, o.offsets, o.order, s.num_tokens * o.top_k, o.num_experts,
                          o.top_k, o.n, o.k, o.gather, o.scatter, o.act};
-    // bfloat16 operands in whole 16-byte pieces: the tensor-core form (the activation in its epilogue)
-    // many rows an expert: the tcgen05 kernel, on tiles of 128 rows
+    // bfloat16 operands in whole 16-byte pieces: the tensor-core forms (the activation in their epilogues)
     const std::string& how = ex.choice("grouped_linear");
     auto* t5 = (GroupedTcgen05Fn)ex.find("grouped_tcgen05");
     auto* fits = (GroupedFitsFn)ex.find("grouped_tcgen05_supports");
     if (t5 && fits && o.x_dtype == LLME_DT_BF16 && o.w_dtype == LLME_DT_BF16 && ex.choice("linear") != "plain" && (!o.gather || o.rows) &&
-        (how == "tcgen05" || (how == "auto" && (long long)a.pairs >= GROUPED_ROWS * o.num_experts)) && fits(&a, o.out_dtype)) {
+        (how == "tcgen05" || (how == "auto" && ((long long)a.pairs >= GROUPED_ROWS * o.num_experts || !grouped_streams(ex, a)))) && fits(&a, o.out_dtype)) {
         if (o.gather) ++ex.launches;
         return ex.launched(t5(&a, o.rows, o.out_dtype, st), "grouped_tcgen05");
     }

@@ -1,5 +1,6 @@
-"""The grouped product where experts get a few rows: tiles of 8 and 16 pairs (and, from 16 pairs an expert on, of 64), experts with no,
-one and one more row than a tile, more experts than a warp looks at in one go, odd sizes; against 64 bits."""
+"""The grouped product where experts get a few rows: streamed in tiles of 8 and 16 pairs (and, from 16 pairs an expert on, tiles of 64), and
+on tcgen05, which serves many experts from the first row on; experts with no, one and one more row than a tile, more experts than a
+warp looks at in one go, odd sizes; against 64 bits."""
 import pytest
 import torch
 
@@ -15,10 +16,11 @@ DEV = "cuda:0"
     ([5, 2, 0, 7], 2, 2048, 2048), ([20, 33, 64, 65], 2, 130, 200)])
 @pytest.mark.parametrize("act", [None, "silu", "relu2", "gelu"])
 @pytest.mark.parametrize("gather,scatter", [(True, False), (False, True)])
-def test_few_rows(rows, top, n, k, act, gather, scatter):
+@pytest.mark.parametrize("kernel", ["mma", "tcgen05"])
+def test_few_rows(rows, top, n, k, act, gather, scatter, kernel):
     from llmengine_b200.kernels.ops import CudaOps
     ops, g = CudaOps(torch.device(DEV)), torch.Generator(device=DEV).manual_seed(sum(rows) + n)
-    ops.choose("grouped_linear", "mma")
+    ops.choose("grouped_linear", kernel)
     E, pairs = len(rows), -(-sum(rows) // top) * top
     rows = rows[:-1] + [rows[-1] + pairs - sum(rows)]                    # whole tokens
     T = pairs // top
@@ -29,7 +31,8 @@ def test_few_rows(rows, top, n, k, act, gather, scatter):
     n_out = n // 2 if act == "silu" else n
     dtype = torch.bfloat16 if gather else torch.float32
     out, mid, plan = torch.full((pairs, n_out), 7.0, dtype=dtype, device=DEV), torch.empty(pairs, n, dtype=torch.bfloat16, device=DEV), Plan()
-    plan.grouped_linear(x=x, w=w, out=out, offsets=offsets, order=order, top_k=top, gather=gather, scatter=scatter, mid=mid, act=act)
+    plan.grouped_linear(x=x, w=w, out=out, offsets=offsets, order=order, top_k=top, gather=gather, scatter=scatter, mid=mid, act=act,
+                        rows=torch.empty(pairs, k, dtype=torch.bfloat16, device=DEV) if gather else None)
     ops.compile(plan).run(StepBatch.bare(T, torch.device(DEV)))
     torch.cuda.synchronize()
     for e in range(E):

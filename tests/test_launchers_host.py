@@ -159,3 +159,30 @@ def test_shares_are_fewer_where_the_scratch_memory_is_small(compiled):
     assert most > 3
     assert _window_step(compiled, 2, 16, 4, 0, 0, 8000, 1).splits == 1
     assert _window_step(compiled, 2, 16, 4, 0, 0, 8000, 65536 + 2 * 16 * 3 * 130).splits == 3
+
+
+@pytest.mark.parametrize("experts,top,n,k,tokens,streams", [
+    # the faster of the two kernels as measured, from a quarter to three and a half rows an expert; one whose products are small is
+    # streamed, one of many short rows is not
+    (8, 2, 2048, 2048, 1, True), (8, 2, 4096, 2048, 14, True), (16, 4, 2048, 1024, 6, True), (32, 4, 2048, 2048, 8, True), (32, 4, 4096, 2048, 8, True),
+    (32, 4, 4096, 2048, 20, True), (64, 8, 1024, 2048, 24, True), (128, 8, 1024, 2048, 8, True), (32, 4, 2048, 1024, 24, False), (64, 6, 2048, 1024, 27, False),
+    (64, 8, 2048, 512, 16, False), (128, 8, 1024, 2048, 40, False), (128, 8, 2048, 512, 4, False), (128, 8, 2048, 512, 48, False), (128, 8, 1536, 2048, 48, False),
+    (64, 4, 2048, 1536, 32, False),
+    # from four rows on
+    (8, 2, 2048, 2048, 16, False), (32, 4, 4096, 2048, 32, False), (128, 8, 2048, 512, 1000, False)])
+def test_grouped_products_of_few_rows(compiled, experts, top, n, k, tokens, streams):
+    e = _Executor(compiled("executor"))
+    P, far = c_void_p, 1 << 24
+    e.kernel("grouped_tcgen05", P, P, c_int, P)
+    e.kernel("grouped_tcgen05_supports", P, c_int, result=1)
+    e.kernel("grouped_linear_tc", P, c_int, c_int, c_int, P)
+    op = e.ex.GroupedLinearOp()
+    for name in ("x", "w", "out", "offsets", "order", "mid", "rows"):
+        setattr(op, name, far)
+    gather = k == 2048 and (experts, n) != (8, 2048)                 # (the gate|up product; the down product's rows lie side by side)
+    op.ldx = op.ldw = op.k = k
+    op.ldo, op.n, op.w_expert, op.num_experts, op.top_k, op.x_dtype, op.w_dtype, op.gather, op.act = n, n, n * k, experts, top, 1, 1, int(gather), int(gather)
+    step = e.ex.Step()
+    step.num_tokens = step.num_requests = tokens
+    e.run(e.ex.OP_GROUPED_LINEAR, op, step)
+    assert list(e.given)[-1] == ("grouped_linear_tc" if streams else "grouped_tcgen05")
