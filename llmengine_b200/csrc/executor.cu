@@ -661,6 +661,12 @@ int latent_splits(const LlmeExecutor& ex, int requests, int nh, long long max_ct
     return s < 1 ? 1 : (int)s;
 }
 
+// Portions whose contexts are all within half a key tile of the tcgen05 kernels stay on the warp-level ones: a block's set-up there takes
+// longer than the whole attention (whole layers, 16 / 32 heads, tcgen05 and warp-level us: latent, one request of 8 tokens 31.0 / 46.4 and 26.9 /
+// 42.8, 32 tokens 34.4 / 57.4 and 31.8 / 50.3, 64 tokens 35.0 / 58.2 and 34.4 / 55.4, 96 tokens 38.0 / 61.1 and 40.3 / 60.0; window, 8 tokens
+// 21.1 / 34.2 and 18.6 / 32.1, 64 tokens 26.4 / 42.2 and 23.6 / 38.6, 96 tokens 26.0 / 43.6 and 25.9 / 42.9).
+bool short_portions(const LlmeStep& s) { return s.max_portion_ctx > 0 && s.max_portion_ctx <= 64; }
+
 int op_latent_attention(LlmeExecutor& ex, const LlmeLatentAttentionOp& o, const LlmeStep& s, cudaStream_t st) {
     if (s.num_tokens <= 0) return 0;
     if (o.group < 0 || o.group >= s.num_groups) return ex.fail("latent attention: the step has no cache group %d", o.group);
@@ -686,10 +692,11 @@ int op_latent_attention(LlmeExecutor& ex, const LlmeLatentAttentionOp& o, const 
         if (s.num_portion > 0) {
             f.rows = s.portion_rows; f.n_rows = s.num_portion; f.splits = 1;
             // On tcgen05 where the latent size and the pages allow it: 128 keys of 128 (token, head) rows take a pair of blocks 3.2 us there, 32
-            // keys of 64 rows 4.3 us of the warp-level kernel's block, so it is ahead from the shortest portion on.
+            // keys of 64 rows 4.3 us of the warp-level kernel's block, so it is ahead from the shortest portion on, but for contexts of its
+            // first half tile (short_portions).
             auto* pair = (LatentPairFn)ex.find_hd("latent_pair", o.rank);
             auto* pair_fits = (LatentPairFitsFn)ex.find_hd("latent_pair_supports", o.rank);
-            if (pair && pair_fits && ex.choice("attention.portion") == "tcgen05" && pair_fits(o.rot, g.page_size) && aligned16(o.q, o.cache, o.out)) {
+            if (pair && pair_fits && ex.choice("attention.portion") == "tcgen05" && !short_portions(s) && pair_fits(o.rot, g.page_size) && aligned16(o.q, o.cache, o.out)) {
                 if (int rc = ex.launched(pair(&f, (long long)s.num_tokens * o.nh, o.cache_rows, o.sink, o.rot, s.max_portion_len, st), "latent_pair")) return rc;
             } else if (int rc = ex.launched(tc(&f, o.sink, o.rot, s.max_portion_len, st), "latent_attention_tc")) return rc;
         }
@@ -825,7 +832,7 @@ int window_attend(LlmeExecutor& ex, const LlmeWindowAttentionOp& o, const LlmeSt
         // 134 us of the warp-level kernel for 1,900 tokens of 16 / 4 heads of 128)
         const int rep = o.nh / o.nkv, ps = g.page_size;
         auto* big = o.dk == o.dv && o.value_share <= 1 ? (AttnTcFn)ex.find_hd("attention_tc", o.dk) : nullptr;
-        if (s.num_portion > 0 && big && ex.choice("attention.portion") == "tcgen05" && ps >= 8 && (ps <= 128 ? 128 % ps == 0 : ps % 128 == 0) && 128 % rep == 0 &&
+        if (s.num_portion > 0 && big && ex.choice("attention.portion") == "tcgen05" && !short_portions(s) && ps >= 8 && (ps <= 128 ? 128 % ps == 0 : ps % 128 == 0) && 128 % rep == 0 &&
             aligned16(o.q, o.cache, o.out)) {
             LlmeTcAttnArgs a = {o.out, o.cache, s.portion_rows, s.cu_q_lens, s.ctx_lens, s.state_slots, g.block_tables, g.max_blocks, s.num_portion, o.nh,
                                 o.nkv, ps, o.window, o.scale, 0.0f, 0.0f, 0.0f, o.sink, o.keep_first, o.softcap};

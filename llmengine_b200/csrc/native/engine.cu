@@ -1045,7 +1045,7 @@ private:
             int *tok = m, *pos = m + T_cap, *treq = m + 2 * T_cap, *slot = m + 3 * T_cap, *lrows = m + 4 * T_cap;
             int* cu = m + 5 * T_cap;
             int *ctx = cu + R_cap + 1, *slots = ctx + R_cap, *first = slots + R_cap, *dec = first + R_cap, *por = dec + R_cap;
-            int a = 0, nl = 0, nd = 0, np = 0, max_portion = 0, max_decode_ctx = 0;
+            int a = 0, nl = 0, nd = 0, np = 0, max_portion = 0, max_portion_ctx = 0, max_decode_ctx = 0;
             cu[0] = 0;
             for (int r = 0; r < R; ++r) {
                 const StepEntry& e = entries[r];
@@ -1069,6 +1069,7 @@ private:
                 } else {
                     por[np++] = r;
                     max_portion = std::max(max_portion, n);
+                    max_portion_ctx = std::max(max_portion_ctx, s + n);
                 }
             }
             CUDA_OK(cudaMemcpyAsync(meta_dev_, pinned_, meta_len_ * 4, cudaMemcpyHostToDevice, stream_));
@@ -1078,7 +1079,7 @@ private:
             }
             LlmeStep st = {};
             st.num_tokens = T; st.num_requests = R; st.num_logit_rows = NL; st.num_decode = nd; st.num_portion = np;
-            st.max_portion_len = max_portion; st.max_decode_ctx = max_decode_ctx;
+            st.max_portion_len = max_portion; st.max_decode_ctx = max_decode_ctx; st.max_portion_ctx = max_portion_ctx;
             int* d = meta_dev_;
             st.token_ids = d; st.positions = d + T_cap; st.token_request = d + 2 * T_cap; st.logit_rows = d + 4 * T_cap;
             int* dcu = d + 5 * T_cap;

@@ -61,6 +61,8 @@ typedef struct LlmeStep {
     void* blas;                /* cublasHandle_t bound to `stream` by the caller, or NULL: the executor's own */
     int num_groups;
     LlmeStepGroup groups[LLME_MAX_GROUPS];
+    int max_portion_ctx;       /* longest context among the requests with several tokens (0: not known); it decides between kernels of
+                                  the same result, so a replay may meet others */
 } LlmeStep;
 
 typedef int (*LlmeCallFn)(void* user, const LlmeStep* step, cudaStream_t stream);

@@ -61,6 +61,13 @@ def test_single_tokens_of_other_sizes(rank, rot, heads, ctx):
     run(rank, rot, heads, 16, 0, True, [(ctx, 1), (0, 1), (ctx // 2, 1)], ranges=True)
 
 
+@pytest.mark.parametrize("lens", [[(0, 64), (30, 2), (0, 1)], [(0, 65)], [(0, 3)], [(0, 64), (900, 1)]])
+@pytest.mark.parametrize("sink", [True, False])
+def test_short_portions(lens, sink):
+    """Up to 64 keys the warp-level kernel serves them, whatever single tokens beside them see."""
+    run(512, 64, 16, 16, 0, sink, lens)
+
+
 @pytest.mark.parametrize("heads,sink", [(16, True), (16, False), (32, True)])
 def test_portions_are_no_further_off_than_the_warp_level_kernel(heads, sink):
     """Both round the probabilities to bfloat16.  The warp-level kernel takes them relative to the row's true maximum, whose probability is
@@ -72,7 +79,7 @@ def test_portions_are_no_further_off_than_the_warp_level_kernel(heads, sink):
 
 def test_a_single_key_beside_a_sink():
     """A row of one key: its probability is 1 / (1 + exp(sink - score)), and nothing but the result is rounded where the key leads."""
-    heads, T = 16, 60
+    heads, T = 16, 100
     out, want, lead = run(512, 64, heads, 16, 1, True, [(0, T)], single=True)
     assert int(lead.sum()) > 100
     bound = (2.0 ** -8 + 1e-4) * want.abs()                  # half a unit of the last of eight digits, and the 32-bit exponentials

@@ -40,6 +40,12 @@ def test_window_attention(H, G, d, page, window, first, sink, cap, norm, rot, in
     run(H, G, d, page, window, first, sink, cap, norm, rot, interleaved, lens)
 
 
+@pytest.mark.parametrize("lens", [[(0, 64), (30, 2), (0, 1)], [(0, 65)], [(0, 3)], [(0, 64), (900, 1)]])
+def test_short_portions(lens):
+    """Up to 64 keys the warp-level kernel serves them, whatever single tokens beside them see."""
+    run(16, 4, 128, 16, 40, 3, True, 0.0, True, 64, False, lens)
+
+
 @pytest.mark.parametrize("floats", [0, 1, 65536 + 4 * 16 * 2 * 130])
 def test_any_scratch_memory_is_enough(floats):
     """As many shares of a context as their partial results find room for, one at least."""

@@ -186,3 +186,33 @@ def test_grouped_products_of_few_rows(compiled, experts, top, n, k, tokens, stre
     step.num_tokens = step.num_requests = tokens
     e.run(e.ex.OP_GROUPED_LINEAR, op, step)
     assert list(e.given)[-1] == ("grouped_linear_tc" if streams else "grouped_tcgen05")
+
+
+@pytest.mark.parametrize("ctx,decode_ctx,short", [(64, 0, True), (2, 0, True), (64, 900, True), (65, 0, False), (3000, 10, False), (0, 0, False)])
+def test_short_portions_stay_on_the_warp_level_kernels(compiled, ctx, decode_ctx, short):
+    """By the longest context among the requests with several tokens, where the step tells it."""
+    P, far = c_void_p, 1 << 24
+    e = _Executor(compiled("executor"))
+    step = e.ex.Step()
+    step.num_tokens, step.num_requests, step.num_portion, step.max_portion_len = 40, 2, 2, 30
+    step.max_portion_ctx, step.max_decode_ctx, step.num_decode, step.num_groups = ctx, decode_ctx, 1 if decode_ctx else 0, 1
+    step.groups[0] = e.ex.StepGroup(far, far, 1024, 16, 0)
+    e.kernel("latent_post", P, c_int, P)
+    e.kernel("latent_attention_tc/512", P, P, c_int, c_int, P)
+    e.kernel("latent_attention_tc_fits/512", c_int, result=1)
+    e.kernel("latent_pair/512", P, c_longlong, c_longlong, P, c_int, c_int, P)
+    e.kernel("latent_pair_supports/512", c_int, c_int, result=1)
+    op = e.ex.LatentAttentionOp()
+    op.kv_in = op.c_gain = op.q = op.out = op.cache = far
+    op.dtype, op.nh, op.rank, op.rot, op.scale, op.cache_rows = 1, 16, 512, 64, 0.1, 1 << 16
+    e.run(e.ex.OP_LATENT_ATTENTION, op, step)
+    assert ("latent_pair/512" in e.given) != short
+    step.groups[0].window = 100
+    e.kernel("window_post", P, c_int, P)
+    e.kernel("window_attention_tc/128x128", P, c_int, c_int, P)
+    e.kernel("attention_tc/128", P, c_longlong, c_longlong, P, c_int, P)
+    op = e.ex.WindowAttentionOp()
+    op.q_in = op.k_in = op.v_in = op.q = op.out = op.cache = op.sink = far
+    op.dtype, op.nh, op.nkv, op.dk, op.dv, op.window, op.scale, op.amplitude, op.cache_pages, op.value_share = 1, 16, 4, 128, 128, 100, 0.1, 1.0, 4096, 1
+    e.run(e.ex.OP_WINDOW_ATTENTION, op, step)
+    assert ("attention_tc/128" in e.given) != short
