@@ -20,8 +20,9 @@
 //               (A load takes its warp some 100 cycles to issue, and pages of 16 tokens are 68 loads a tile: one warp alone needed
 //               7,800 cycles a tile, the matrix instructions 3,700.)
 //
-// Measured (a 2,000-token prompt, 16 heads on rows of 512 + 64, pages of 16): 122 us, against 454 us of the warp-level kernel, whose time
-// went into the fragments that every warp re-read from shared memory.  A key tile takes 5,900 cycles: 36 instructions of 33 cycles and
+// Measured (a 2,000-token prompt, 16 heads on rows of 512 + 64, pages of 16): about 129 us, against 454 us of the warp-level kernel, whose time
+// went into the fragments that every warp re-read from shared memory.  A key tile takes some 6,200 cycles (5,900 while the reference only
+// moved by 2^8): 36 instructions of 33 cycles and
 // 16 of 65 are 2,200 of them, waits for loads 1,900: the ring covers 1,800 cycles, about what a load needs from L2 to its barrier.
 //
 // Every wait is bounded; one that gives up sets the error flag (llme_latent_pair_status()) and the block drains and returns.

@@ -7,9 +7,11 @@
 //
 //   warp 0      producer: TMA loads of the Q tiles (3-D boxes: tokens x heads of the group x 64 columns) and,
 //               page by page through the block table, of the K and V tiles (128-byte swizzle, two stages
-//               each, one load per lane, the keys one tile ahead of the values).  A page that holds keys
-//               beyond what the block may see is copied by hand instead, with those rows zeroed, so that
-//               stale memory (NaN included) never reaches the tensor cores.
+//               each, one load per lane, the keys one tile ahead of the values).  The box that the request
+//               ends in is copied by hand instead, with the rows behind its last token zeroed, so that
+//               stale memory (NaN included) never reaches the tensor cores.  What a held page contains before
+//               that token must be finite, whether the block's rows see it or not: their scores are masked, and
+//               a probability of zero times such a value must be zero.
 //   warp 1      issues the matrix instructions, alternating between the two Q tiles so that the tensor pipe
 //               works for one while the softmax of the other runs: S_t = Q_t K^T (128 x 128 x HEAD_DIM) into
 //               the tile's score columns of tensor memory, and O_t += P_t V (128 x HEAD_DIM x 128) into its
@@ -288,7 +290,8 @@ struct Barriers {
 };
 
 // EXT: with a sink, kept first positions or a cap on the scores (a form of its own, so that plain attention does not carry them).  Two
-// prompts of 1,900 tokens in all, 16 / 4 heads of 128, a window of 1,024 and four kept positions take 47 us, 134 us on the warp-level kernel.
+// prompts of 1,900 tokens in all, 16 / 4 heads of 128, a window of 1,024 and four kept positions take 58 us, 134 us on the warp-level kernel
+// (47 us with probabilities before the tile's maximum, as in plain attention, which rounds the largest of them too).
 template <bool EXT>
 __global__ void __launch_bounds__(THREADS, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,

@@ -691,7 +691,7 @@ int op_latent_attention(LlmeExecutor& ex, const LlmeLatentAttentionOp& o, const 
         f.page_size = g.page_size; f.scale = o.scale; f.window = o.window;
         if (s.num_portion > 0) {
             f.rows = s.portion_rows; f.n_rows = s.num_portion; f.splits = 1;
-            // On tcgen05 where the latent size and the pages allow it: 128 keys of 128 (token, head) rows take a pair of blocks 3.2 us there, 32
+            // On tcgen05 where the latent size and the pages allow it: 128 keys of 128 (token, head) rows take a pair of blocks 3.4 us there, 32
             // keys of 64 rows 4.3 us of the warp-level kernel's block, so it is ahead from the shortest portion on, but for contexts of its
             // first half tile (short_portions).
             auto* pair = (LatentPairFn)ex.find_hd("latent_pair", o.rank);
@@ -828,7 +828,7 @@ int window_attend(LlmeExecutor& ex, const LlmeWindowAttentionOp& o, const LlmeSt
         f.table_rows = s.state_slots; f.block_tables = g.block_tables; f.max_blocks = g.max_blocks; f.nh = o.nh; f.nkv = o.nkv;
         f.page_size = g.page_size; f.window = o.window; f.keep_first = o.keep_first; f.scale = o.scale; f.softcap = o.softcap;
         f.value_share = o.value_share;
-        // prompt portions over keys and values of one width: the tcgen05 kernel with a sink, kept first positions and a cap (47 us against
+        // prompt portions over keys and values of one width: the tcgen05 kernel with a sink, kept first positions and a cap (58 us against
         // 134 us of the warp-level kernel for 1,900 tokens of 16 / 4 heads of 128)
         const int rep = o.nh / o.nkv, ps = g.page_size;
         auto* big = o.dk == o.dv && o.value_share <= 1 ? (AttnTcFn)ex.find_hd("attention_tc", o.dk) : nullptr;
@@ -1006,6 +1006,8 @@ int op_moe_route(LlmeExecutor& ex, const LlmeMoeRouteOp& o, const LlmeStep& s, c
 // Rows an expert gets in the mean, from which on the tcgen05 kernel is ahead: its tiles of 128 rows are mostly padding then, but the
 // experts' matrices are what takes the time, and it reads them once.  A mixture of 4 of 32 experts of 2,048 x 2,048 (bfloat16, whole layer),
 // this kernel against the warp-level ones: 16 tokens (2 rows) 153 / 143 us, 32 (4 rows) 175 / 186, 96 177 / 220, 250 185 / 446, 500 198 / 395.
+// Of other mixtures, products alone at four rows, this kernel / streaming us: 8 experts 2048 x 2048 21 / 14, 16 experts 2048 x 1024 18 / 20,
+// 64 experts 1024 x 2048 58 / 55, 128 experts 1024 x 2048 99 / 119, 128 experts 2048 x 512 46 / 159.
 constexpr long long GROUPED_ROWS = 4;
 
 // Below that: the weight-streaming form or the tcgen05 kernel, whichever these estimates of their times (us) give less.  A streaming block

@@ -12,8 +12,9 @@
 //
 // 16 x 16 threads hold TM x TN outputs each, as packed pairs of neighbouring columns (fma.rn.f32x2: one instruction, each half
 // rounds as fmaf does); operands lie in shared memory k by k, two stages, the next one on its way through registers.
-// Bound by the multiply-adds: 300 x 11008 x 2048 takes 376 us and 300 x 2048 x 5504 216 us (36 and 31 TFLOP/s of 74; 2,048 rows: 50
-// and 44); one block per 64 x 64 tile with 4 x 4 outputs a thread, whatever the shape, took 675 and 617 us.
+// Bound by shared memory, whose path is 87 to 89 % busy while the multiply-adds fill 55 % of theirs: 300 x 11008 x 2048 takes 376 us and
+// 300 x 2048 x 5504 206 us (36 and 33 TFLOP/s of 74; 2,048 rows: 50 and 44); one block per 64 x 64 tile with 4 x 4 outputs a thread,
+// whatever the shape, took 675 and 617 us.
 // Up to 32 rows a third form streams the weights (further down).
 //
 // Reference counterparts: sgemm_nt_kernel (src/runtime/kernels/cuda_kernels.cu:282-294,
@@ -361,8 +362,11 @@ int sm_count() {
 }
 
 // Which tile, and whether a cluster shares its segments: the least number of rounds times a block's work.  A block's rate relative to
-// that of 128 x 128 outputs: what its operands cost
-// beside the multiply-adds (two 16-byte loads from shared memory for 64 of them, one and a quarter for 8).
+// that of 128 x 128 outputs (`rate`): what its operands cost beside the multiply-adds (two 16-byte loads from shared memory for 64 of
+// them, one and a quarter for 8).  A round is a block an SM, although two find room there: two share its multiply-adds and its shared
+// memory.  The 64 and 32 values of k stand for a cluster's and a further segment's sums.  All of it is an estimate: over 90 sizes (33 to
+// 2,048 rows on 512 to 11,008 outputs of 600 to 5,504 values) its choice is within 5 % of the best of the eight forms in 82, and
+// at worst 23 % behind (256 x 2048 x 5504: 251 us against 204); 300 x 11008 x 2048 takes 376 us so, 365 at best, 402 in tiles of 128.
 template <typename WT>
 int dispatch(const Problem<WT>& g, int batch, cudaStream_t stream) {
     const int bm[4] = {128, 64, 64, 16}, bn[4] = {128, 128, 64, 128};

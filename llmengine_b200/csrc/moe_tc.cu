@@ -335,8 +335,8 @@ int launch(const LlmeGroupedArgs& a, cudaStream_t s) {
     LLME_LAUNCH_STATUS();
 }
 
-// Rows an expert in the mean (the routing itself is on the device): tiles of 8 pairs, of 16, or of 64 through shared memory.  (From 4 rows on
-// the tcgen05 kernel serves what it can; without it 16-pair tiles take that mixture 266 us at 124 tokens and 327 us at 160, 64-pair
+// Rows an expert in the mean (the routing itself is on the device): tiles of 8 pairs, of 16, or of 64 through shared memory.  (From 4 rows on,
+// and below where that is estimated to be faster, the tcgen05 kernel serves what it can; without it 16-pair tiles take that mixture 266 us at 124 tokens and 327 us at 160, 64-pair
 // tiles 279 us at 400.)
 constexpr long long SKINNY_8 = 4, SKINNY_16 = 16;
 

@@ -439,8 +439,10 @@ LLME_API int llme_latent_post(const LlmeLatentPostArgs* args, int dtype, cudaStr
     if (a.rot > 0 && (!a.inv_freq || a.rot_dims <= 0 || a.rot_dims % 2 || a.rot_dims > a.rot))
         LLME_REFUSE("latent_post: %d rotated coordinates of %d need frequencies and an even count", a.rot_dims, a.rot);
     const int threads = 128;
-    // (up to 256 tokens the blocks below, of which a token has several, are through before a table is formed: 24 tokens of 16 heads
-    // take a layer 90.3 us so, 92.1 us in pieces)
+    // Alone, 16 / 32 heads with 512 + 64, us, below / in pieces: 64 tokens 3.5 / 3.5 and 3.2 / 3.7, 128 3.4 / 3.6 and 3.3 / 3.7, 256 3.9 / 4.6 and
+    // 3.5 / 3.9; from 257 on, where the form below has one block a token for the queries instead of eight, 6.3 / 11.1 and 3.5 / 4.0, 600 11.0 / 20.1
+    // and 4.3 / 5.6.  Between two others few tokens are better served by the many blocks, which are through before a table is formed
+    // (a layer of 24 tokens 90.3 us so, 92.1 us in pieces).
     if (a.tokens > 256 && latent_pieces(a, dtype) && (a.gain_dtype == LLME_BF16 || a.gain_dtype == LLME_F32)) {
         const dim3 pieces_grid(a.tokens);
         const size_t smem = (size_t)(a.rot > 0 ? a.rot_dims : 0) * sizeof(float);

@@ -421,7 +421,7 @@ int llme_executor_register(LlmeExecutor*, const char* name, void* entry_point);
  *   "linear_swiglu":     "fused" | "unfused"
  *   "attention.portion": "tcgen05" | "mma" | "plain"
  *   "attention.decode":  "fused" | "split" | "plain"
- *   "grouped_linear":    "auto" | "tcgen05" | "mma"                 (bfloat16: many rows an expert / all / none)
+ *   "grouped_linear":    "auto" | "tcgen05" | "mma"                 (bfloat16, on tcgen05: many rows an expert or much to read / all / none)
  *   "delta_rule":        "blocks" | "tokens"                        (portions: eight tokens at a time / one after the other)
  *   "*":                 "fast" | "plain"                           (all of the above at once)
  * Returns 0, or -1 for an unknown operation or variant. */
