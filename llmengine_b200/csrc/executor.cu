@@ -304,7 +304,7 @@ int product(LlmeExecutor& ex, const LlmeStep& step, const void* x, long long ldx
             int w_dtype, void* out, long long ldo, int out_dtype, int M, int N, int K, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (x_dtype == LLME_DT_F32) {
-        // the 32-bit path: this package's FMA kernel, never a reduced-precision mode
+        // the 32-bit path: this package's own kernel, never a reduced-precision mode
         auto* f = (GemmF32Fn)ex.find("gemm_f32");
         if (!f) return ex.fail("linear: no 32-bit product kernel is registered");
         if (out_dtype != LLME_DT_F32) return ex.fail("linear: a 32-bit product writes 32-bit output");

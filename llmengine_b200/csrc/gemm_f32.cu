@@ -1,6 +1,7 @@
-// True 32-bit matrix product C[M,N] = A[M,K] * W[N,K]^T on the CUDA cores (FMA, no
-// tensor cores, no reduced-precision mode).  It is the matrix product of the whole
-// 32-bit path and the plain twin that the tensor-core kernels are checked against.
+// True 32-bit matrix product C[M,N] = A[M,K] * W[N,K]^T.  It is the matrix product of the whole 32-bit path and the plain twin that the
+// tensor-core kernels are checked against.  Float weights whose rows begin on 16 bytes go to the tensor cores in pieces that keep all 24
+// bits (gemm_f32_tcgen05.cuh); everything else (bfloat16 weights, batches of products, fewer than 512 values, odd row strides) is multiplied
+// and added on the CUDA cores, in the forms below.
 //
 // K is cut into S segments of equal length, S = K / 1024 between 1 and 8; every output element adds the products of a
 // segment in the order of k, and then the segments' sums in their order.  S depends on K alone, so a row's result does not
@@ -19,6 +20,8 @@
 //
 // Reference counterparts: sgemm_nt_kernel (src/runtime/kernels/cuda_kernels.cu:282-294,
 // one thread per output, no tiling) and the cublasSgemm call of sgemm_nt_cublas (:892-908).
+#include <cuda.h>
+
 #include "common.cuh"
 
 LLME_API const char* llme_last_error() { return llme_error_buffer(); }
@@ -395,6 +398,8 @@ int dispatch(const Problem<WT>& g, int batch, cudaStream_t stream) {
     LLME_REFUSE("gemm_f32: M = %d needs more than 65535 grid rows", g.M);
 }
 
+#include "gemm_f32_tcgen05.cuh"
+
 template <typename WT>
 int product(const float* A, const WT* W, float* C, int M, int N, int K, long long lda, long long ldw, long long ldc, int batch, long long sa,
             long long sw, long long sc, cudaStream_t stream) {
@@ -405,6 +410,10 @@ int product(const float* A, const WT* W, float* C, int M, int N, int K, long lon
     g.vec_a = (uintptr_t)A % 16 == 0 && lda % 4 == 0 && sa % 4 == 0;
     g.vec_w = (uintptr_t)W % (4 * sizeof(WT)) == 0 && ldw % 4 == 0 && sw % 4 == 0;
     g.vec_c = (uintptr_t)C % 16 == 0 && ldc % 4 == 0 && sc % 4 == 0;
+    if (sizeof(WT) == 4 && batch == 1 && split::takes(N, K, A, W, lda, ldw)) {
+        split::Args a = {A, (const float*)W, C, M, N, K, 0, 0, 0, g.vec_c, lda, ldw, ldc};
+        return split::product(a, stream);
+    }
     // Few rows stream the weights: 32 rows take 73 and 50 us against 119 and 74 in tiles, 48 rows (two passes) 115 and 95 against 121
     // and 78.  (Copies of four values need the alignment; the tiles take everything.)
     if (M <= FEW_ROWS && g.vec_a && g.vec_w) {
@@ -438,3 +447,6 @@ LLME_API int llme_gemm_nt_f32(const float* A, const void* W, int w_dtype, float*
                               long long lda, long long ldw, long long ldc, cudaStream_t stream) {
     return llme_gemm_nt_f32_batched(A, W, w_dtype, C, M, N, K, lda, ldw, ldc, 1, 0, 0, 0, stream);
 }
+
+// 0, or where a bounded wait of the tensor-core form gave up.
+LLME_API int llme_gemm_f32_status() { LLME_TAKE_STATUS(split::g_status); }

@@ -42,3 +42,47 @@ def test_a_batch_of_products():
         ops.compile(plan).run(StepBatch.bare(T, torch.device(DEV)))
         want = torch.einsum("tbk,bnk->tbn", x.double(), w.double())
         assert float((out.double() - want).norm() / want.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("N,K,pad", [(64, 512, 0), (65, 577, 3), (129, 1030, 2), (300, 1024, 0), (2048, 5500, 4), (11008, 640, 0), (19000, 512, 0)])
+def test_float_weights_on_the_tensor_cores(N, K, pad):
+    """Around the edges of tiles, chunks of 64 values and segments.  An output's chunk is 24 instructions that may each cut off a last place of
+    what has been added so far, 2^-23 of sum |x w| at most; the chunks' and segments' sums round once each, 2^-24, and the pieces leave out
+    less than 2^-25 of each product, three times."""
+    from llmengine_b200.kernels.ops import CudaOps
+    ops, g = CudaOps(torch.device(DEV)), torch.Generator(device=DEV).manual_seed(N + K)
+    x = torch.randn(260, K + pad, generator=g, device=DEV)[:, :K]
+    w = torch.randn(N, K + pad, generator=g, device=DEV)[:, :K]
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    bound = (2 * 24 + K / 64 + 5 + 1.5) * 2.0 ** -24 * size
+    full = None
+    for M in (260, 1, 8, 16, 17, 32, 33, 48, 112, 113, 225):
+        out = torch.full((M, N + 4), 5.0, device=DEV)
+        ops.linear(x[:M], w, out[:, :N])
+        assert bool((out[:, N:] == 5.0).all())
+        full = out[:, :N] if full is None else full
+        assert bool(((out[:, :N].double() - want[:M]).abs() <= bound[:M]).all()), M
+        assert torch.equal(out[:, :N], full[:M]), M
+    assert int(ops._lib("gemm_f32").llme_gemm_f32_status()) == 0
+
+
+def test_no_number_where_32_bits_give_none_and_only_there():
+    """Infinities, NaN, values next to the largest (which bfloat16 rounds up to infinity), sums that overflow, and tiny rows."""
+    from llmengine_b200.kernels.ops import CudaOps
+    ops, g = CudaOps(torch.device(DEV)), torch.Generator(device=DEV).manual_seed(3)
+    for M in (20, 150):
+        x, w = torch.randn(M, 1024, generator=g, device=DEV), torch.randn(256, 1024, generator=g, device=DEV) * 0.02
+        x[3, 5], x[4, 7], x[5, 9], w[7, 11], w[8, 12] = float("inf"), float("nan"), 3.4e38, -float("inf"), 3.4e38
+        x[6] *= 1e-30
+        x[9] = 0.0
+        x[10] *= 1e36
+        x[11, 20], x[11, 21], w[9, 20], w[9, 21] = 3e38, 3e38, 1.0, 1.0
+        out = torch.empty(M, 256, device=DEV)
+        ops.linear(x, w, out)
+        exact = x.double() @ w.double().t()
+        large = exact.abs() >= (2 - 2.0 ** -24) * 2.0 ** 127               # from here on a value rounds to infinity in 32 bits
+        assert torch.equal(out.isnan(), exact.isnan())
+        assert torch.equal(out.isinf(), exact.isinf() | large) and bool((torch.sign(out) == torch.sign(exact))[large].all())
+        rest = torch.isfinite(exact) & ~large
+        size = x.double().abs() @ w.double().abs().t()
+        assert bool(((out.double() - exact).abs() <= (2 * 24 + 1024 + 8) * 2.0 ** -24 * size)[rest].all())
