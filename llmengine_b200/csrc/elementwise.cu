@@ -719,49 +719,61 @@ __global__ void qkv_post_vec_kernel(QkvArgs a) {
     }
 }
 
-// Many tokens, bfloat16 in and out, a head size of 32, 64, 128 or 256: a warp takes one token and a run of
-// heads.  What belongs to the token (its position's cos/sin values, its cache slot, the gains) is loaded once
-// per warp instead of once per head, a lane holds 4 + 4 values of a head (8-byte loads and stores), and the
-// 32 lanes cover 32 / LPH heads at a time, so that a head costs about half the instructions of the kernel above.
-constexpr int QKV_WIDE_ITERS = 2;      // head groups per warp
+// Many tokens, bfloat16 in and out, a head size of 32, 64, 128 or 256: a warp takes one token and a run of heads.  What belongs to the
+// token (its position's cosines and sines, its cache slot) is loaded once per warp instead of once per head; a lane holds 8 + 8 values
+// of a head (16-byte loads and stores), and all loads of its heads are on their way before the first is used.
+// Bound by latency, not by the 8 TB/s that its 50 MB would take at 2,048 tokens of 32 + 8 + 8 heads of 128: position and slot are looked
+// up in front of what depends on them, so a warp should have many bytes in flight.  That size takes 11.4 us, 17.5 with 8-byte pieces and twice
+// as many warps a token; 2,800 tokens of 16 + 4 + 4 heads 8.5 us and 12.5 (three heads a lane: 11.7 us, one: 14.3 us at the first size).
+constexpr int QKV_WIDE_ITERS = 2;      // heads a lane takes part in
 constexpr int QKV_WIDE_WARPS = 8;      // = tokens per block
 
-__device__ __forceinline__ void bf16x4_to_f32(uint2 v, float (&f)[4]) {
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
-    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
-    f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+__device__ __forceinline__ void bf16x8_to_f32(uint4 v, float (&f)[8]) {
+    const unsigned w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 p = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+        f[2 * i] = p.x;
+        f[2 * i + 1] = p.y;
+    }
 }
-__device__ __forceinline__ uint2 f32_to_bf16x4(const float (&f)[4]) {
-    uint2 v;
-    *reinterpret_cast<__nv_bfloat162*>(&v.x) = __floats2bfloat162_rn(f[0], f[1]);
-    *reinterpret_cast<__nv_bfloat162*>(&v.y) = __floats2bfloat162_rn(f[2], f[3]);
-    return v;
+__device__ __forceinline__ uint4 f32_to_bf16x8(const float (&f)[8]) {
+    unsigned w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<__nv_bfloat162*>(&w[i]) = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+    return make_uint4(w[0], w[1], w[2], w[3]);
 }
-template <typename G> __device__ __forceinline__ void load_gain4(const G* p, float (&g)[4]);
-template <> __device__ __forceinline__ void load_gain4<float>(const float* p, float (&g)[4]) {
-    const float4 v = *reinterpret_cast<const float4*>(p);
-    g[0] = v.x; g[1] = v.y; g[2] = v.z; g[3] = v.w;
+__device__ __forceinline__ void load8(const float* p, float (&g)[8]) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w; g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w;
 }
-template <> __device__ __forceinline__ void load_gain4<__nv_bfloat16>(const __nv_bfloat16* p, float (&g)[4]) {
-    bf16x4_to_f32(*reinterpret_cast<const uint2*>(p), g);
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&g)[8]) { bf16x8_to_f32(*reinterpret_cast<const uint4*>(p), g); }
+
+// WHOLE: rows begin on 16 bytes; else (a row stride that is a multiple of four values only) on 8.
+template <bool WHOLE>
+__device__ __forceinline__ uint4 load_bf16x8(const __nv_bfloat16* p) {
+    if (WHOLE) return *reinterpret_cast<const uint4*>(p);
+    const uint2 a = reinterpret_cast<const uint2*>(p)[0], b = reinterpret_cast<const uint2*>(p)[1];
+    return make_uint4(a.x, a.y, b.x, b.y);
 }
 
-template <typename G, int LPH>
+template <typename G, int LPH, bool WHOLE>
 __global__ void __launch_bounds__(QKV_WIDE_WARPS * 32, 4) qkv_post_wide_kernel(QkvArgs a) {
     pdl_launch_dependents();   // the next kernel may be scheduled while this one runs
     pdl_wait();                // everything below reads or writes what earlier kernels touch
     typedef __nv_bfloat16 bf16;
     constexpr int HPW = 32 / LPH;                  // heads the warp's lanes cover at a time
-    constexpr int HD = LPH * 8, HALF = HD / 2;
+    constexpr int HD = LPH * 16, HALF = HD / 2;
     const int lane = threadIdx.x & 31;
     const int t = (int)blockIdx.x * QKV_WIDE_WARPS + (int)(threadIdx.x >> 5);
     if (t >= a.tokens) return;
     const int heads = a.nh + 2 * a.nkv;
-    const int d = 4 * (lane % LPH);                // this lane's values: d .. d+3 and HALF+d .. HALF+d+3
+    const int d = 8 * (lane % LPH);                // this lane's values: d .. d+7 and HALF+d .. HALF+d+7
     const int h0 = (int)blockIdx.y * (HPW * QKV_WIDE_ITERS) + lane / LPH;
 
-    // the heads first (the loads that take longest), then what belongs to the token
-    uint2 lo[QKV_WIDE_ITERS], hi[QKV_WIDE_ITERS];
+    int pos = a.cos_sin ? a.positions[t] : 0;
+    const int slot = a.cache ? a.slot_mapping[t] : -1;
+    uint4 lo[QKV_WIDE_ITERS], hi[QKV_WIDE_ITERS];
 #pragma unroll
     for (int it = 0; it < QKV_WIDE_ITERS; ++it) {
         const int h = h0 + it * HPW;
@@ -769,93 +781,81 @@ __global__ void __launch_bounds__(QKV_WIDE_WARPS * 32, 4) qkv_post_wide_kernel(Q
         if (h < a.nh) { if (a.q_in) src = (const bf16*)a.q_in + (size_t)t * a.q_stride + (size_t)h * HD; }
         else if (h < a.nh + a.nkv) { if (a.k_in) src = (const bf16*)a.k_in + (size_t)t * a.k_stride + (size_t)(h - a.nh) * HD; }
         else if (h < heads) { if (a.v_in) src = (const bf16*)a.v_in + (size_t)t * a.v_stride + (size_t)(h - a.nh - a.nkv) * HD; }
-        lo[it] = make_uint2(0u, 0u); hi[it] = make_uint2(0u, 0u);
+        lo[it] = make_uint4(0u, 0u, 0u, 0u); hi[it] = make_uint4(0u, 0u, 0u, 0u);
         if (src) {
-            lo[it] = *reinterpret_cast<const uint2*>(src + d);
-            hi[it] = *reinterpret_cast<const uint2*>(src + HALF + d);
+            lo[it] = load_bf16x8<WHOLE>(src + d);
+            hi[it] = load_bf16x8<WHOLE>(src + HALF + d);
         }
     }
-    float co[4] = {1.0f, 1.0f, 1.0f, 1.0f}, si[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float co[8], si[8];
     if (a.cos_sin) {
-        int pos = a.positions[t];
         pos = pos < 0 ? 0 : (pos >= a.max_positions ? a.max_positions - 1 : pos);   // the host refuses such positions
         const float* cs = a.cos_sin + (size_t)pos * HD;
-        load_gain4<float>(cs + d, co);
-        load_gain4<float>(cs + HALF + d, si);
+        load8(cs + d, co);
+        load8(cs + HALF + d, si);
     }
-    float qg0[4], qg1[4], kg0[4], kg1[4];
-    if (a.q_gain) { load_gain4<G>((const G*)a.q_gain + d, qg0); load_gain4<G>((const G*)a.q_gain + HALF + d, qg1); }
-    if (a.k_gain) { load_gain4<G>((const G*)a.k_gain + d, kg0); load_gain4<G>((const G*)a.k_gain + HALF + d, kg1); }
     bf16* cache_row = nullptr;                     // the token's place in the cache: key of head 0
     size_t kv_step = 0, head_step = 0;
-    if (a.cache) {
-        const int slot = a.slot_mapping[t];
-        if (slot >= 0) {
-            const int page = slot / a.page_size, off = slot - page * a.page_size;
-            head_step = (size_t)a.page_size * HD;
-            kv_step = (size_t)a.nkv * head_step;
-            cache_row = (bf16*)a.cache + (size_t)page * 2 * kv_step + (size_t)off * HD;
-        }
+    if (slot >= 0) {
+        const int page = slot / a.page_size, off = slot - page * a.page_size;
+        head_step = (size_t)a.page_size * HD;
+        kv_step = (size_t)a.nkv * head_step;
+        cache_row = (bf16*)a.cache + (size_t)page * 2 * kv_step + (size_t)off * HD;
     }
 
 #pragma unroll
     for (int it = 0; it < QKV_WIDE_ITERS; ++it) {
         const int h = h0 + it * HPW;
         const bool is_q = h < a.nh, is_k = !is_q && h < a.nh + a.nkv, is_v = !is_q && !is_k && h < heads;
-        float x0[4], x1[4];
-        bf16x4_to_f32(lo[it], x0);
-        bf16x4_to_f32(hi[it], x1);
+        float x0[8], x1[8];
+        bf16x8_to_f32(lo[it], x0);
+        bf16x8_to_f32(hi[it], x1);
         // every lane takes part in the sums, whatever its head is
         float ss = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) ss += x0[i] * x0[i] + x1[i] * x1[i];
+        for (int i = 0; i < 8; ++i) ss += x0[i] * x0[i] + x1[i] * x1[i];
 #pragma unroll
         for (int o = LPH / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         if (is_v) {
             if (cache_row && a.v_in) {
                 bf16* dst = cache_row + kv_step + (size_t)(h - a.nh - a.nkv) * head_step;
-                *reinterpret_cast<uint2*>(dst + d) = lo[it];
-                *reinterpret_cast<uint2*>(dst + HALF + d) = hi[it];
+                *reinterpret_cast<uint4*>(dst + d) = lo[it];
+                *reinterpret_cast<uint4*>(dst + HALF + d) = hi[it];
             }
-            continue;
-        }
-        if (!(is_q || is_k) || !(is_q ? a.q_in : a.k_in)) continue;
-        if (is_q ? a.q_gain != nullptr : a.k_gain != nullptr) {
-            const float rinv = 1.0f / sqrtf(ss / (float)HD + a.eps);
+        } else if ((is_q || is_k) && (is_q ? a.q_in : a.k_in)) {
+            const G* gain = (const G*)(is_q ? a.q_gain : a.k_gain);
+            if (gain) {
+                const float rinv = 1.0f / sqrtf(ss / (float)HD + a.eps);
+                float g[8];
+                load8(gain + d, g);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                x0[i] = (x0[i] * rinv) * (is_q ? qg0[i] : kg0[i]);
-                x1[i] = (x1[i] * rinv) * (is_q ? qg1[i] : kg1[i]);
-            }
-        }
-        if (a.cos_sin) {
+                for (int i = 0; i < 8; ++i) x0[i] = (x0[i] * rinv) * g[i];
+                load8(gain + HALF + d, g);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float u = x0[i], v = x1[i];
-                x0[i] = u * co[i] - v * si[i];
-                x1[i] = u * si[i] + v * co[i];
+                for (int i = 0; i < 8; ++i) x1[i] = (x1[i] * rinv) * g[i];
+            }
+            if (a.cos_sin) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float u = x0[i], v = x1[i];
+                    x0[i] = u * co[i] - v * si[i];
+                    x1[i] = u * si[i] + v * co[i];
+                }
+            }
+            const uint4 o0 = f32_to_bf16x8(x0), o1 = f32_to_bf16x8(x1);
+            bf16* out = is_q ? (a.q_out ? (bf16*)a.q_out + ((size_t)t * a.nh + h) * HD : nullptr)
+                             : (a.k_out ? (bf16*)a.k_out + ((size_t)t * a.nkv + (h - a.nh)) * HD : nullptr);
+            if (out) {
+                *reinterpret_cast<uint4*>(out + d) = o0;
+                *reinterpret_cast<uint4*>(out + HALF + d) = o1;
+            }
+            if (is_k && cache_row) {
+                bf16* dst = cache_row + (size_t)(h - a.nh) * head_step;
+                *reinterpret_cast<uint4*>(dst + d) = o0;
+                *reinterpret_cast<uint4*>(dst + HALF + d) = o1;
             }
         }
-        const uint2 o0 = f32_to_bf16x4(x0), o1 = f32_to_bf16x4(x1);
-        if (is_q) {
-            if (a.q_out) {
-                bf16* dst = (bf16*)a.q_out + ((size_t)t * a.nh + h) * HD;
-                *reinterpret_cast<uint2*>(dst + d) = o0;
-                *reinterpret_cast<uint2*>(dst + HALF + d) = o1;
-            }
-        } else {
-            const int head = h - a.nh;
-            if (a.k_out) {
-                bf16* dst = (bf16*)a.k_out + ((size_t)t * a.nkv + head) * HD;
-                *reinterpret_cast<uint2*>(dst + d) = o0;
-                *reinterpret_cast<uint2*>(dst + HALF + d) = o1;
-            }
-            if (cache_row) {
-                bf16* dst = cache_row + (size_t)head * head_step;
-                *reinterpret_cast<uint2*>(dst + d) = o0;
-                *reinterpret_cast<uint2*>(dst + HALF + d) = o1;
-            }
-        }
+        __syncwarp();
     }
 }
 
@@ -863,8 +863,9 @@ template <typename G, int LPH>
 static void launch_qkv_wide_lph(const QkvArgs& a, cudaStream_t s) {
     const int heads = a.nh + 2 * a.nkv;
     const int per_warp = (32 / LPH) * QKV_WIDE_ITERS;
-    llme_launch(qkv_post_wide_kernel<G, LPH>, dim3((unsigned)((a.tokens + QKV_WIDE_WARPS - 1) / QKV_WIDE_WARPS), (unsigned)((heads + per_warp - 1) / per_warp)),
-                dim3(QKV_WIDE_WARPS * 32), 0, s, a);
+    const dim3 grid((unsigned)((a.tokens + QKV_WIDE_WARPS - 1) / QKV_WIDE_WARPS), (unsigned)((heads + per_warp - 1) / per_warp)), block(QKV_WIDE_WARPS * 32);
+    if ((a.q_stride | a.k_stride | a.v_stride) % 8 == 0) llme_launch(qkv_post_wide_kernel<G, LPH, true>, grid, block, 0, s, a);
+    else llme_launch(qkv_post_wide_kernel<G, LPH, false>, grid, block, 0, s, a);
 }
 
 // Whether the wide kernel takes this call (and then launches it): bfloat16 in and out is the caller's business.
@@ -872,19 +873,18 @@ template <typename G>
 static bool launch_qkv_wide(const QkvArgs& a, cudaStream_t s) {
     const int heads = a.nh + 2 * a.nkv;
     if (a.hd != 32 && a.hd != 64 && a.hd != 128 && a.hd != 256) return false;
-    const int groups = (heads + (256 / a.hd) * QKV_WIDE_ITERS - 1) / ((256 / a.hd) * QKV_WIDE_ITERS);
-    if (groups > 65535) return false;
-    if ((long long)a.tokens * groups < 148LL * 16) return false;                // few tokens: a warp per (token, head)
+    if (heads > 65535) return false;
+    if ((long long)a.tokens * heads * a.hd < 148LL * 16 * 512) return false;    // few tokens: a warp per (token, head)
     if ((a.q_stride | a.k_stride | a.v_stride) & 3) return false;
     const uintptr_t ptrs = (uintptr_t)a.q_in | (uintptr_t)a.k_in | (uintptr_t)a.v_in | (uintptr_t)a.q_gain |
                            (uintptr_t)a.k_gain | (uintptr_t)a.cos_sin | (uintptr_t)a.q_out | (uintptr_t)a.k_out |
                            (uintptr_t)a.cache;
     if (ptrs % 16) return false;
     switch (a.hd) {
-        case 32: launch_qkv_wide_lph<G, 4>(a, s); break;
-        case 64: launch_qkv_wide_lph<G, 8>(a, s); break;
-        case 128: launch_qkv_wide_lph<G, 16>(a, s); break;
-        default: launch_qkv_wide_lph<G, 32>(a, s); break;
+        case 32: launch_qkv_wide_lph<G, 2>(a, s); break;
+        case 64: launch_qkv_wide_lph<G, 4>(a, s); break;
+        case 128: launch_qkv_wide_lph<G, 8>(a, s); break;
+        default: launch_qkv_wide_lph<G, 16>(a, s); break;
     }
     return true;
 }
