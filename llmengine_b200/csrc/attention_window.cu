@@ -399,6 +399,171 @@ __global__ void __launch_bounds__(512) window_post_rows_kernel(LlmeWindowPostArg
     }
 }
 
+// The same where a head is 64, 128 or 256 values and rows lie on 16 bytes: `W` warps a token, up to ten pieces of eight values a lane, all
+// requested before the first is used and kept in registers; a rotated piece finds its partner in another lane of the head.  No piece goes
+// through shared memory, whose two further passes and barriers bound the form above: 1,900 tokens of 16 + 4 heads of 128 take 11.6 us, 15.8 there.
+// Bound by instructions (the exchanges of the rotation most of all): as few warps a token as hold it are fastest (two 15.8 us, four 21.7 us).
+constexpr int POST_PIECES = 10, POST_WARPS = 8;
+template <typename T> struct Eight;
+template <> struct Eight<float> {
+    float4 a, b;
+    __device__ __forceinline__ void load(const float* p) { a = ((const float4*)p)[0]; b = ((const float4*)p)[1]; }
+    __device__ __forceinline__ void values(float (&v)[8]) const { v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w; }
+    static __device__ __forceinline__ void store(float* p, const float (&v)[8]) {
+        ((float4*)p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+        ((float4*)p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+    }
+};
+template <> struct Eight<__nv_bfloat16> {
+    uint4 raw;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { raw = *(const uint4*)p; }
+    __device__ __forceinline__ void values(float (&v)[8]) const {
+        const unsigned w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 f = __bfloat1622float2(*(const __nv_bfloat162*)&w[i]);
+            v[2 * i] = f.x;
+            v[2 * i + 1] = f.y;
+        }
+    }
+    static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&v)[8]) {
+        unsigned w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) *(__nv_bfloat162*)&w[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        *(uint4*)p = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+};
+
+template <typename I, typename T, int LPH>                           // LPH lanes hold a head
+__global__ void __launch_bounds__(32 * POST_WARPS) window_post_warps_kernel(LlmeWindowPostArgs a, int W) {
+    constexpr int DK = 8 * LPH;
+    __shared__ float2 part[POST_WARPS];
+    __shared__ __align__(16) float turns[POST_WARPS][DK];           // a warp's cosines and sines, formed once each
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = warp % W, t = blockIdx.x * (POST_WARPS / W) + warp / W;
+    const bool here = t < a.tokens;
+    const int dv = a.dv, ps = a.page_size, half = a.inv_freq ? a.rot_dims >> 1 : 0, d = 8 * (lane % LPH);
+    const int slot = (here && a.cache && a.slot_mapping && a.k_in) ? a.slot_mapping[t] : -1;
+    const int position = here && half ? a.positions[t] : 0;
+    const int qp = a.nh * LPH, pieces = here ? qp + (slot >= 0 ? a.nkv * LPH : 0) : 0, nv = value_heads(a.nkv, a.value_share);
+    const I* q = (const I*)a.q_in + (size_t)t * a.q_stride;
+    const I* k = (const I*)a.k_in + (size_t)t * a.k_stride;
+    Eight<I> x[POST_PIECES];
+#pragma unroll
+    for (int i = 0; i < POST_PIECES; ++i) {
+        const int p = (i * W + w) * 32 + lane;
+        if (p < pieces) x[i].load(p < qp ? q + 8 * p : k + 8 * (p - qp));
+    }
+    const int page = slot >= 0 ? slot / ps : 0, off = slot - page * ps;
+    T* kpage = (T*)a.cache + (size_t)page * page_values(a.nkv, nv, ps, DK, dv);
+    if (slot >= 0) {                                                 // the values, as they are
+        const I* v = (const I*)a.v_in + (size_t)t * a.v_stride;
+        T* vpage = kpage + (size_t)a.nkv * ps * DK + (size_t)off * dv;
+        for (int j = 8 * (w * 32 + lane); j < nv * dv; j += 8 * 32 * W) {
+            const int g = j / dv;
+            Eight<I> y;
+            float f[8];
+            y.load(v + j);
+            y.values(f);
+            Eight<T>::store(vpage + (size_t)g * ps * dv + (j - g * dv), f);
+        }
+    }
+    for (int i = lane; i < half; i += 32) {
+        float s, c;
+        sincosf((float)position * a.inv_freq[i], &s, &c);
+        turns[warp][i] = c * a.amplitude;
+        turns[warp][half + i] = s * a.amplitude;
+    }
+    __syncwarp();
+    // those of this lane's place in a head, the same for all its pieces; the sine as the partner is multiplied with it
+    const bool turned = d < 2 * half;
+    float co[8], si[8];
+    if (turned)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int i = a.interleaved ? (d + e) >> 1 : (d < half ? d : d - half) + e;
+            co[e] = turns[warp][i];
+            si[e] = (a.interleaved ? !(e & 1) : d < half) ? -turns[warp][half + i] : turns[warp][half + i];
+        }
+    float sq = 0.0f, sk = 0.0f;
+#pragma unroll
+    for (int i = 0; i < POST_PIECES; ++i) {
+        const int p = (i * W + w) * 32 + lane;
+        if (p >= pieces) continue;
+        float v[8], ss = 0.0f;
+        x[i].values(v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
+        if (p < qp) sq += ss; else sk += ss;
+    }
+    sq = warp_sum(sq);
+    sk = warp_sum(sk);
+    if (W > 1) {
+        if (lane == 0) part[warp] = make_float2(sq, sk);
+        __syncthreads();
+        sq = sk = 0.0f;
+        for (int o = 0; o < W; ++o) {
+            sq += part[warp - w + o].x;
+            sk += part[warp - w + o].y;
+        }
+    }
+    const float rq = a.q_gain ? 1.0f / sqrtf(sq / (float)(a.nh * DK) + a.eps) : 1.0f;
+    const float rk = a.k_gain ? 1.0f / sqrtf(sk / (float)(a.nkv * DK) + a.eps) : 1.0f;
+    const int partner = half / 8;                                    // lanes to the partner of a pair of halves: a power of two
+#pragma unroll
+    for (int i = 0; i < POST_PIECES; ++i) {
+        const int p = (i * W + w) * 32 + lane;
+        if ((i * W + w) * 32 >= pieces) break;                       // (the whole warp)
+        const bool mine = p < pieces, is_q = p < qp;
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = 0.0f;
+        if (mine) x[i].values(v);
+        const float* gain = is_q ? a.q_gain : a.k_gain;
+        if (mine && gain) {
+            const float r = is_q ? rq : rk;
+            Eight<float> g;
+            float f[8];
+            g.load(gain + 8 * (is_q ? p : p - qp));
+            g.values(f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = (v[e] * r) * f[e];
+        }
+        if (half) {
+            float o[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[e] = a.interleaved ? v[e ^ 1] : __shfl_xor_sync(0xffffffffu, v[e], partner);
+            if (turned)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = v[e] * co[e] + o[e] * si[e];
+        }
+        if (mine) {
+            const int h = p / LPH;
+            if (is_q) Eight<T>::store((T*)a.q_out + (size_t)t * a.nh * DK + 8 * p, v);
+            else Eight<T>::store(kpage + ((size_t)(h - a.nh) * ps + off) * DK + d, v);
+        }
+    }
+}
+
+template <typename I, typename T>
+static bool launch_post_warps(const LlmeWindowPostArgs& a, cudaStream_t s) {
+    const int half = a.inv_freq ? a.rot_dims / 2 : 0, pieces = (a.nh + a.nkv) * (a.dk / 8);
+    const bool fits = (a.dk == 64 || a.dk == 128 || a.dk == 256) && a.dv % 8 == 0 && pieces <= 32 * POST_WARPS * POST_PIECES &&
+                      (!half || (a.interleaved ? half % 4 == 0 : half % 8 == 0 && (half & (half - 1)) == 0)) &&
+                      (a.q_stride | a.k_stride | a.v_stride) * (long long)sizeof(I) % 16 == 0 &&
+                      ((uintptr_t)a.q_in | (uintptr_t)a.k_in | (uintptr_t)a.v_in | (uintptr_t)a.q_out | (uintptr_t)a.cache | (uintptr_t)a.q_gain | (uintptr_t)a.k_gain) % 16 == 0;
+    if (!fits) return false;
+    // as few warps a token as hold it, more where the tokens alone do not give every scheduler two
+    int W = 1;
+    while (W < POST_WARPS && (pieces > 32 * W * POST_PIECES || ((long long)a.tokens * W < 148 * 8 && pieces > 32 * W))) W *= 2;
+    const dim3 grid((a.tokens + POST_WARPS / W - 1) / (POST_WARPS / W)), block(32 * POST_WARPS);
+    if (a.dk == 64) llme_launch(window_post_warps_kernel<I, T, 8>, grid, block, 0, s, a, W);
+    else if (a.dk == 128) llme_launch(window_post_warps_kernel<I, T, 16>, grid, block, 0, s, a, W);
+    else llme_launch(window_post_warps_kernel<I, T, 32>, grid, block, 0, s, a, W);
+    return true;
+}
+
 template <typename I, typename T>
 static bool launch_post_rows(const LlmeWindowPostArgs& a, cudaStream_t s) {
     const size_t smem = ((size_t)(a.nh + a.nkv) * a.dk + (a.inv_freq ? a.rot_dims : 0)) * sizeof(float);
@@ -478,6 +643,9 @@ LLME_API int llme_window_post(const LlmeWindowPostArgs* args, int dtype, cudaStr
         else LLME_REFUSE("window_post: unsupported dtype %d", dtype);
         LLME_LAUNCH_STATUS();
     }
+    if (dtype == LLME_F32 ? launch_post_warps<float, float>(a, stream)
+                          : dtype == LLME_BF16 && (wide_in ? launch_post_warps<float, __nv_bfloat16>(a, stream) : launch_post_warps<__nv_bfloat16, __nv_bfloat16>(a, stream)))
+        LLME_LAUNCH_STATUS();
     if (dtype == LLME_F32 ? launch_post_rows<float, float>(a, stream)
                           : dtype == LLME_BF16 && (wide_in ? launch_post_rows<float, __nv_bfloat16>(a, stream) : launch_post_rows<__nv_bfloat16, __nv_bfloat16>(a, stream)))
         LLME_LAUNCH_STATUS();
