@@ -19,7 +19,12 @@
 // the inverse N of the unit lower triangular I + A, and B N, so that u = N r and o = G S0^T q + (B N) r: lane i of a column forms
 // u_i and o_i from the eight r's, and nothing is left to be solved in sequence.  No quotient of decays is ever formed, so a decay of
 // zero is harmless.  A block at a portion's end is filled up with tokens that change nothing (k = q = 0, b = 0, a = 1); how a
-// prompt is cut into steps changes the order of the sums and nothing else.
+// prompt is cut into steps changes the order of the sums and nothing else.  Long portions of heads with 128 rows go 64 tokens at a time
+// on the tensor cores instead (delta_chunks.cuh).
+#include <cuda.h>
+
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernel_args.h"
 
@@ -486,6 +491,8 @@ int launch_tile(const LlmeDeltaArgs& a, int vec_state, cudaStream_t s) {
     LLME_LAUNCH_STATUS();
 }
 
+#include "delta_chunks.cuh"
+
 bool rows_of_16(const void* p, long long stride, int n) { return (uintptr_t)p % 16 == 0 && stride % 4 == 0 && n % 4 == 0; }
 
 int check(const LlmeDeltaArgs& a) {
@@ -520,6 +527,7 @@ LLME_API int llme_delta_portions(const LlmeDeltaArgs* args, cudaStream_t stream)
     if (a.n_rows <= 0) return 0;
     if (int rc = check(a)) return rc;
     if (!a.unit || !a.coef || ((uintptr_t)a.unit | (uintptr_t)a.coef) % 16) LLME_REFUSE("delta_rule: portions need their workspace");
+    if (chunks::takes(a)) return chunks::launch(a, stream);
     const dim3 blocks(a.tokens / BLOCK + a.requests + 1, (a.qk_groups + PREPARE_WARPS - 1) / PREPARE_WARPS);
     llme_launch(delta_prepare_kernel, blocks, dim3(32 * PREPARE_WARPS), 0, stream, a);
     const int vs = rows_of_16(a.state, a.state_stride, a.n);
@@ -533,3 +541,6 @@ LLME_API int llme_delta_portions(const LlmeDeltaArgs* args, cudaStream_t stream)
     if (a.n <= 256) return launch_tile<16, 4, 1, 4, 3>(a, vs, stream);
     return launch_tile<32, 4, 1, 4, 2>(a, vs, stream);
 }
+
+// 0, or where a bounded wait of the form that takes 64 tokens at a time gave up.
+LLME_API int llme_delta_status() { LLME_TAKE_STATUS(chunks::g_status); }

@@ -942,7 +942,7 @@ int op_delta_rule(LlmeExecutor& ex, const LlmeDeltaRuleOp& o, const LlmeStep& s,
     if (!step || !portions) return ex.fail("no delta_rule kernels are registered");
     LlmeDeltaArgs a = {o.q, o.k, o.v, o.ldq, o.ldk, o.ldv, o.write, o.forget, o.ld_gates, o.dt_bias, o.a_log, o.q_scale, o.unit_eps, o.state,
                        o.state_stride, o.out, o.ldo, s.cu_q_lens, s.state_slots, nullptr, s.num_requests, s.num_requests, s.num_tokens, o.heads,
-                       o.n, o.p, o.qk_groups, o.unit, o.coef};
+                       o.n, o.p, o.qk_groups, o.unit, o.coef, o.coef_floats};
     if (ex.choice("delta_rule") == "tokens") return ex.launched(step(&a, st), "delta_step");      // every request, token after token
     if (s.num_portion > 0) {
         const long long n4 = (o.n + 3) / 4 * 4, blocks = s.num_tokens / 8 + s.num_requests + 1;

@@ -428,7 +428,7 @@ class Engine:
     # libraries whose kernels wait with a limit -> what says whether a wait gave up (and forgets it)
     _STATUS = {"gemm_tcgen05": "llme_gemm_tc_status", "moe_tcgen05": "llme_grouped_tcgen05_status", "attention_tc": "llme_attention_tc_status",
                "attention_latent_tc": "llme_latent_attention_tc_status", "attention_latent_tcgen05": "llme_latent_pair_status",
-               "gemm_f32": "llme_gemm_f32_status"}
+               "gemm_f32": "llme_gemm_f32_status", "delta_rule": "llme_delta_status"}
 
     def check_kernels(self) -> None:
         """Raise if a bounded wait inside a kernel has given up since the last call (synchronises the device)."""

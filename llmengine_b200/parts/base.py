@@ -296,11 +296,13 @@ class Runtime:
     def delta_workspace(self, heads: int, qk_heads: int, n: int) -> Tuple[torch.Tensor, torch.Tensor]:
         """What the delta rule over portions works from: the unit queries and keys of every token ([tokens, 2 * qk_heads * n'],
         n' = n rounded up to whole groups of four), and per block of eight tokens of a request and head the 160 numbers that
-        its columns share (one buffer each for all layers; blocks are numbered floor(first token / 8) + place of
-        the request in the step + block of the request)."""
+        its columns share (one buffer each for all layers; blocks are numbered floor(first token / 8) + place of the request in the
+        step + block of the request).  Portions of 256 tokens or more on average may instead go by chunks of 64 tokens where a head is
+        128, with 8,448 numbers per chunk and head; chunks are numbered alike, by place among the portions."""
         n4 = (n + 3) // 4 * 4
-        blocks = self.max_tokens // 8 + self.max_requests + 1
-        self._delta_coef_floats = max(getattr(self, "_delta_coef_floats", 0), blocks * heads * 160)
+        blocks, chunks = self.max_tokens // 8 + self.max_requests + 1, self.max_tokens // 64 + self.max_tokens // 256 + 1
+        need = max(blocks * heads * 160, chunks * heads * 8448 if n == 128 and self.max_tokens >= 256 else 0)
+        self._delta_coef_floats = max(getattr(self, "_delta_coef_floats", 0), need)
         return (self.workspace("delta_unit", 2 * qk_heads * n4, torch.float32),
                 self.buffer("delta_coef", 1, self._delta_coef_floats, torch.float32, exact=True).view(-1))
 
