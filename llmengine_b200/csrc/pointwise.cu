@@ -145,7 +145,7 @@ __global__ void sigmoid_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ a, l
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const float2 x = __bfloat1622float2(h[e]), y = __bfloat1622float2(z[e]);
-            h[e] = __floats2bfloat162_rn(x.x * __frcp_rn(1.0f + __expf(-y.x)) * scale, x.y * __frcp_rn(1.0f + __expf(-y.y)) * scale);
+            h[e] = __floats2bfloat162_rn(x.x * reciprocal_above_one(1.0f + __expf(-y.x)) * scale, x.y * reciprocal_above_one(1.0f + __expf(-y.y)) * scale);
         }
         o[j] = v;
     }

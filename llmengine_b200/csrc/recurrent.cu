@@ -972,7 +972,7 @@ __global__ void __launch_bounds__(128) gated_norm_fours_kernel(LlmeGatedNormArgs
                 if (a.gate) {
                     // (a result that goes to bfloat16 takes the hardware's exponential and reciprocal)
                     const float z = gate[k][i][e];
-                    const float s = sizeof(T) == 2 ? __frcp_rn(1.0f + __expf(-z)) : 1.0f / (1.0f + expf(-z));
+                    const float s = sizeof(T) == 2 ? reciprocal_above_one(1.0f + __expf(-z)) : 1.0f / (1.0f + expf(-z));
                     f = a.gate_act == 1 ? s : z * s;
                 }
                 u[k][i][e] = u[k][i][e] * rinv * w[e] * f * a.scale;

@@ -19,7 +19,7 @@ constexpr int MOST_STREAMS = 16;
 
 // sigmoid(z): in the 32-bit path, and where the products take bfloat16 (a few units in the last place of 32-bit)
 __device__ __forceinline__ float gate_of(float z, float) { return 1.0f / (1.0f + expf(-z)); }
-__device__ __forceinline__ float gate_of(float z, bf16) { return __frcp_rn(1.0f + __expf(-z)); }
+__device__ __forceinline__ float gate_of(float z, bf16) { return reciprocal_above_one(1.0f + __expf(-z)); }
 
 template <typename T> __device__ __forceinline__ float4 load4(const T* p);
 template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
