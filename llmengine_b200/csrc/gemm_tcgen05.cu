@@ -226,12 +226,14 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& map_x, const CUt
                         unsigned up[32];
                         tmem_ld_32x32(tmem_row + (unsigned)(BN / 2 + c + half * 32), up);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        auto gates = [&](auto gate) {                 // (which gate it is, asked once and not for every value)
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(v[j])));
-                            const float u = __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[j])));
-                            v[j] = __float_as_uint(gated_mul_bf16(a.pointwise, g, u, a.p0, a.p1));
-                        }
+                            for (int j = 0; j < 32; ++j)
+                                v[j] = __float_as_uint(gate(__bfloat162float(__float2bfloat16_rn(__uint_as_float(v[j]))),
+                                                            __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[j])))));
+                        };
+                        if (a.pointwise == 0) gates([](float g, float u) { return silu_mul_bf16(g, u); });
+                        else gates([&](float g, float u) { return gated_mul_bf16(a.pointwise, g, u, a.p0, a.p1); });
                     } else {
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                         if (a.pointwise == 1) {
