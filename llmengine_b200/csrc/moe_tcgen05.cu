@@ -4,9 +4,13 @@
 // Rows that have to be gathered by token are first written side by side (gather_rows_kernel); from then on a tile of 128 pairs of
 // an expert is a plain box of a matrix, and the pipeline is that of the dense product (gemm_tcgen05.cu): TMA brings 128 x 64
 // pieces of the rows and 256 x 64 pieces of the expert's matrix into shared memory (128-byte swizzle, four stages), one thread
-// issues tcgen05.mma (128 x 256 x 16) into tensor memory, double-buffered, and four warps read the accumulator back, apply the
-// activation and store whole 128-byte pieces of the rows, scattered by pair where asked.  A box at the end of an expert's rows
+// issues tcgen05.mma (128 x 256 x 16) into tensor memory, double-buffered, and eight warps read the accumulator back, apply the
+// activation and store whole 64-byte pieces of the rows, scattered by pair where asked.  A box at the end of an expert's rows
 // runs on into the next expert's: those rows are computed and not stored.  The experts' matrices are one matrix [E n, k].
+//
+// 2,800 pairs of 32 experts, width 2,048, 1,024 outputs: gate and up 56 us, down 31 (64 and 33 with four warps that read back, which took the last
+// tile 11.7 us, half of them for a branch in the gate's reciprocal, and without the set-up under the kernel before).  The 256 tiles of gate and up
+// are 1.7 rounds of the SMs: the first moves 7 TB/s, the second, of 108 SMs, 5.3.
 //
 // Persistent: one block per SM walks over the tiles (expert, 128 rows, columns), which it counts from the routing's offsets.
 // act 1: a tile's 256 accumulator columns are 128 gate rows and the 128 up rows of the same outputs, silu(gate) * up is stored;
@@ -22,8 +26,8 @@ namespace {
 
 #include "umma.cuh"
 
-constexpr int BN = 256, STAGES = 4, MAX_EXPERTS = 1024;
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGING = 4 * 4096;
+constexpr int BN = 256, STAGES = 4, MAX_EXPERTS = 1024, EPILOGUE = 8, BLOCK = 32 * (2 + EPILOGUE);
+constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGING = EPILOGUE * 2048;
 constexpr unsigned TMEM_COLS = 512;
 constexpr size_t SMEM = 1024 + (size_t)STAGES * (A_BYTES + B_BYTES) + STAGING + (2 * STAGES + 4) * 8 + 16 + 2 * (MAX_EXPERTS + 1) * 4;
 static_assert(SMEM <= 232448, "the block's shared memory must fit an SM");
@@ -47,7 +51,7 @@ __device__ __forceinline__ Tile find_tile(const int* starts, const int* offsets,
 }
 
 template <int ACT, typename O>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(BLOCK, 1)
 grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, LlmeGroupedArgs a) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -66,7 +70,6 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
     constexpr int OUT_COLS = ACT == 1 ? BN / 2 : BN;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, E = a.num_experts;
     const int n_out = ACT == 1 ? a.n / 2 : a.n, n_tiles = (n_out + OUT_COLS - 1) / OUT_COLS, k_blocks = (a.k + BK - 1) / BK;
-    for (int e = threadIdx.x; e <= E; e += THREADS) offsets[e] = a.offsets[e];
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full + s, 1);
@@ -74,11 +77,17 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(acc_full + b, 1);
-            mbar_init(acc_empty + b, 4);                           // one arrival per epilogue warp
+            mbar_init(acc_empty + b, EPILOGUE);                    // one arrival per epilogue warp
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)), "r"(TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    pdl_wait();                                                    // (the offsets and the rows come from the kernels before)
+    for (int e = threadIdx.x; e <= E; e += BLOCK) offsets[e] = a.offsets[e];
     __syncthreads();
     if (warp == 0) {                                               // running count of row tiles
         int base = 0;
@@ -94,10 +103,6 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
             base += __shfl_sync(0xffffffffu, sum, 31);
         }
         if (lane == 0) starts[E] = base;
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)), "r"(TMEM_COLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -157,11 +162,12 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
             }
         }
     } else {
-        // ------------------------------------------------------------------ epilogue (warps 2..5)
+        // ------------------------------------------------------------------ epilogue (warps 2..9): a quarter of the rows, every other 64 bytes of them
         const int quarter = warp & 3;               // the TMEM lanes this warp may read: 32 * (warp % 4) ...
-        constexpr int COLS = 128 / (int)sizeof(O);  // output columns per 128-byte piece of a row
+        const int side = (warp - 2) >> 2;
+        constexpr int COLS = 64 / (int)sizeof(O);   // output columns per 64-byte piece of a row
         constexpr int EACH = 16 / (int)sizeof(O);   // and per 16 bytes
-        unsigned char* buf = staging + quarter * 4096;
+        unsigned char* buf = staging + (warp - 2) * 2048;
         O* out = (O*)a.out;
         int i = 0;
         for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
@@ -173,68 +179,66 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
             __syncwarp();
             const unsigned tmem_row = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(b * BN);
 #pragma unroll 1
-            for (int c = 0; c < OUT_COLS; c += COLS) {
+            for (int c = side * 32; c < OUT_COLS; c += 64) {
+                unsigned v[32];
+                tmem_ld_32x32(tmem_row + (unsigned)c, v);
+                if (ACT == 1) {
+                    unsigned up[32];
+                    tmem_ld_32x32(tmem_row + (unsigned)(BN / 2 + c), up);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int half = 0; half < COLS / 32; ++half) {
-                    unsigned v[32];
-                    tmem_ld_32x32(tmem_row + (unsigned)(c + half * 32), v);
-                    if (ACT == 1) {
-                        unsigned up[32];
-                        tmem_ld_32x32(tmem_row + (unsigned)(BN / 2 + c + half * 32), up);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(v[j])));
-                            const float u = __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[j])));
-                            v[j] = __float_as_uint(silu_mul_bf16(g, u));
-                        }
-                    } else {
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        if (ACT == 2) {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(relu2(__uint_as_float(v[j])));
-                        }
-                        if (ACT == 3) {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(gelu_erf(__uint_as_float(v[j])));
-                        }
+                    for (int j = 0; j < 32; ++j) {
+                        const float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(v[j])));
+                        const float u = __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[j])));
+                        v[j] = __float_as_uint(silu_mul_bf16(g, u));
                     }
-                    if (c + COLS >= OUT_COLS && half == COLS / 32 - 1) {     // the tile has left tensor memory
-                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(acc_empty + b);
+                } else {
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (ACT == 2) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(relu2(__uint_as_float(v[j])));
                     }
-                    // row `lane` of the piece; its 16-byte chunk q goes to place q ^ (lane % 8), so that neither side collides
-                    if (sizeof(O) == 4) {
+                    if (ACT == 3) {
 #pragma unroll
-                        for (int q = 0; q < 8; ++q)
-                            *reinterpret_cast<uint4*>(buf + lane * 128 + ((q ^ (lane & 7)) << 4)) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                    } else {
+                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(gelu_erf(__uint_as_float(v[j])));
+                    }
+                }
+                if (c + 64 >= OUT_COLS) {                                    // this warp's part of the tile has left tensor memory
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acc_empty + b);
+                }
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            uint4 pk;
+                for (int part = 0; part < 32 / COLS; ++part) {
+                    // row `lane` of the piece; its 16-byte chunk q goes to place q ^ (lane / 2 % 4), so that neither side collides
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        uint4 pk;
+                        if (sizeof(O) == 4) pk = make_uint4(v[part * 16 + 4 * q], v[part * 16 + 4 * q + 1], v[part * 16 + 4 * q + 2], v[part * 16 + 4 * q + 3]);
+                        else {
                             unsigned* pw = reinterpret_cast<unsigned*>(&pk);
 #pragma unroll
                             for (int e = 0; e < 4; ++e) {
-                                __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[8 * q + 2 * e]), __uint_as_float(v[8 * q + 2 * e + 1]));
+                                __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[(8 * q + 2 * e) & 31]), __uint_as_float(v[(8 * q + 2 * e + 1) & 31]));
                                 pw[e] = *reinterpret_cast<unsigned*>(&h);
                             }
-                            *reinterpret_cast<uint4*>(buf + lane * 128 + (((half * 4 + q) ^ (lane & 7)) << 4)) = pk;
                         }
+                        *reinterpret_cast<uint4*>(buf + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4)) = pk;
                     }
-                }
-                __syncwarp();
-                const int q = lane & 7, col = tl.col0 + c + q * EACH;
+                    __syncwarp();
+                    const int q = lane & 3, col = tl.col0 + c + part * COLS + q * EACH;
 #pragma unroll
-                for (int rr = lane >> 3; rr < 32; rr += 4) {                 // eight lanes store a row's 128 bytes
-                    const int to = __shfl_sync(0xffffffffu, dst, rr);
-                    const uint4 piece = *reinterpret_cast<const uint4*>(buf + rr * 128 + ((q ^ (rr & 7)) << 4));
-                    if (to >= 0 && col < n_out) *reinterpret_cast<uint4*>(out + (size_t)to * a.ldo + col) = piece;
+                    for (int rr = lane >> 2; rr < 32; rr += 8) {             // four lanes store a row's 64 bytes
+                        const int to = __shfl_sync(0xffffffffu, dst, rr);
+                        const uint4 piece = *reinterpret_cast<const uint4*>(buf + rr * 64 + ((q ^ ((rr >> 1) & 3)) << 4));
+                        if (to >= 0 && col < n_out) *reinterpret_cast<uint4*>(out + (size_t)to * a.ldo + col) = piece;
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
             }
         }
     }
+    pdl_launch_dependents();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {
@@ -261,7 +265,7 @@ int launch(const LlmeGroupedArgs& a, const void* x, long long ldx, cudaStream_t 
     auto kernel = grouped_tcgen05_kernel<ACT, O>;
     static LlmeGrants grants;
     if (cudaError_t e = llme_grant_smem(grants, kernel, SMEM)) LLME_REFUSE("grouped_tcgen05: cannot reserve %zu bytes of shared memory: %s", SMEM, cudaGetErrorString(e));
-    kernel<<<sm_count(), THREADS, SMEM, s>>>(mx, mw, a);
+    llme_launch(kernel, dim3(sm_count()), dim3(BLOCK), SMEM, s, mx, mw, a);
     LLME_LAUNCH_STATUS();
 }
 
