@@ -9,10 +9,10 @@
 //   * chunk_prepare_kernel makes what no column of S has a say in, a block per chunk and query/key group: unit vectors, N, B and three
 //     numbers a token, by 32-bit multiply-adds.
 //   * chunk_walk_kernel walks a request's chunks, a block per (32 columns, head): four products a chunk, [K; Q] S, [N; B] r, K^T u' and
-//     [N; B] u, each of 32-bit values split into three bfloat16 pieces (split32.cuh) with sums of at most 128 products in tensor memory.
+//     [N; B] u, each of 32-bit values split into three bfloat16 pieces (split32.cuh) with sums of at most 64 values in tensor memory.
 //     The state stays in 32-bit registers, a row of S a thread.  [K; Q] and [N; B] are first operands in tensor memory; K^T comes from
 //     shared memory with its tokens as the summed side; S, r, u and u' are written there as they lie in the threads, 64-byte rows.
-//     Four warps walk, four split the next chunk's operands, one issues, one copies.
+//     Eight warps walk, eight split the next chunk's operands, one issues, one copies.
 // No quotient of decays is formed.  A chunk at a portion's end is filled up with tokens that change nothing (k = q = 0, b = 0, a = 1).
 // A value that is not finite would reach tokens before its own through the zeros of N and B: a block that meets one in u goes on token by token.
 // Bound by the chain of the four products of a chunk and the exchanges between them, some 6,700 cycles for 64 tokens, behind a preparation
