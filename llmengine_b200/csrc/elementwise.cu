@@ -810,12 +810,21 @@ __global__ void __launch_bounds__(QKV_WIDE_WARPS * 32, 4) qkv_post_wide_kernel(Q
         float x0[8], x1[8];
         bf16x8_to_f32(lo[it], x0);
         bf16x8_to_f32(hi[it], x1);
-        // every lane takes part in the sums, whatever its head is
-        float ss = 0.0f;
+        // Every lane takes part in the sums, whatever its head is.  They are formed as by lanes of 4 + 4 values: two sums of four a lane, added
+        // over the lanes side by side and to one another last.  That is the order in which a head's squares have always been added, and
+        // a sum in another one moves some of the bfloat16 roundings behind it (and with them, layers later, all outputs).
+        float s0 = 0.0f, s1 = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ss += x0[i] * x0[i] + x1[i] * x1[i];
+        for (int i = 0; i < 4; ++i) {
+            s0 += x0[i] * x0[i] + x1[i] * x1[i];
+            s1 += x0[4 + i] * x0[4 + i] + x1[4 + i] * x1[4 + i];
+        }
 #pragma unroll
-        for (int o = LPH / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        for (int o = LPH / 2; o > 0; o >>= 1) {
+            s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+        }
+        const float ss = s0 + s1;
         if (is_v) {
             if (cache_row && a.v_in) {
                 bf16* dst = cache_row + kv_step + (size_t)(h - a.nh - a.nkv) * head_step;

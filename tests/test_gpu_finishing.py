@@ -90,3 +90,24 @@ def test_rows_that_begin_on_eight_bytes(nh, nkv, hd):
                      k_gain=gain, eps=1e-6, cos_sin=table, positions=positions, q_out=out, cache=cache, slot_mapping=positions, page_size=page)
         outs.append((out, cache))
     assert float(outs[0][0].abs().max()) > 0 and torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(32, 8, 128), (16, 4, 256), (40, 20, 64), (60, 30, 32)])
+def test_the_squares_of_a_head_are_added_in_their_order(nh, nkv, hd):
+    """Sums of four pairs (d, hd / 2 + d), then over neighbouring fours from the farthest to the nearest: the order decides some roundings to
+    bfloat16, and with them every output behind the layer.  (Squares of bfloat16 values are exact in 32 bits.)"""
+    from llmengine_b200.kernels.ops import CudaOps
+    ops, g, T, eps = CudaOps(torch.device(DEV)), torch.Generator(device=DEV).manual_seed(hd), 3000, 1e-6
+    n, lanes = (nh + 2 * nkv) * hd, hd // 8
+    rows = torch.randn(T, n, generator=g, device=DEV).to(torch.bfloat16)
+    gain, out = 1 + 0.1 * torch.randn(hd, generator=g, device=DEV), torch.zeros(T, nh * hd, device=DEV, dtype=torch.bfloat16)
+    ops.qkv_post(q_in=rows[:, :nh * hd], k_in=rows[:, nh * hd:(nh + nkv) * hd], v_in=rows[:, (nh + nkv) * hd:], num_heads=nh, num_kv_heads=nkv, head_dim=hd, q_gain=gain,
+                 k_gain=gain, eps=eps, cos_sin=None, positions=torch.arange(T, dtype=torch.int32, device=DEV), q_out=out, cache=None, slot_mapping=None, page_size=16)
+    x = rows[:, :nh * hd].float().view(T, nh, hd)
+    pairs = (x[..., :hd // 2] ** 2 + x[..., hd // 2:] ** 2).view(T, nh, lanes, 4)
+    s = ((pairs[..., 0] + pairs[..., 1]) + pairs[..., 2]) + pairs[..., 3]
+    while s.shape[-1] > 1:
+        half = s.shape[-1] // 2
+        s = s[..., :half] + s[..., half:]
+    want = (x * (1.0 / torch.sqrt(s / hd + torch.tensor(eps, device=DEV)))) * gain
+    assert torch.equal(out, want.to(torch.bfloat16).view(T, nh * hd))
