@@ -437,7 +437,7 @@ template <> struct Eight<__nv_bfloat16> {
 template <typename I, typename T, int LPH>                           // LPH lanes hold a head
 __global__ void __launch_bounds__(32 * POST_WARPS) window_post_warps_kernel(LlmeWindowPostArgs a, int W) {
     constexpr int DK = 8 * LPH;
-    __shared__ float2 part[POST_WARPS];
+    __shared__ float squares[POST_WARPS * POST_PIECES][32];         // sums of squares of a token's pieces, where several warps hold them
     __shared__ __align__(16) float turns[POST_WARPS][DK];           // a warp's cosines and sines, formed once each
     pdl_launch_dependents();
     pdl_wait();
@@ -486,7 +486,10 @@ __global__ void __launch_bounds__(32 * POST_WARPS) window_post_warps_kernel(Llme
             co[e] = turns[warp][i];
             si[e] = (a.interleaved ? !(e & 1) : d < half) ? -turns[warp][half + i] : turns[warp][half + i];
         }
+    // A lane adds every 32nd piece of the token in their order, whichever warps hold them: the sums are not to depend on W, which is chosen
+    // by how many tokens the step has.
     float sq = 0.0f, sk = 0.0f;
+    float (*mine)[32] = squares + (warp - w) * POST_PIECES;
 #pragma unroll
     for (int i = 0; i < POST_PIECES; ++i) {
         const int p = (i * W + w) * 32 + lane;
@@ -495,19 +498,18 @@ __global__ void __launch_bounds__(32 * POST_WARPS) window_post_warps_kernel(Llme
         x[i].values(v);
 #pragma unroll
         for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
-        if (p < qp) sq += ss; else sk += ss;
+        if (W > 1) mine[i * W + w][lane] = ss;
+        else if (p < qp) sq += ss;
+        else sk += ss;
+    }
+    if (W > 1) {
+        __syncthreads();
+        for (int p = lane; p < pieces; p += 32) {
+            if (p < qp) sq += mine[p >> 5][lane]; else sk += mine[p >> 5][lane];
+        }
     }
     sq = warp_sum(sq);
     sk = warp_sum(sk);
-    if (W > 1) {
-        if (lane == 0) part[warp] = make_float2(sq, sk);
-        __syncthreads();
-        sq = sk = 0.0f;
-        for (int o = 0; o < W; ++o) {
-            sq += part[warp - w + o].x;
-            sk += part[warp - w + o].y;
-        }
-    }
     const float rq = a.q_gain ? 1.0f / sqrtf(sq / (float)(a.nh * DK) + a.eps) : 1.0f;
     const float rk = a.k_gain ? 1.0f / sqrtf(sk / (float)(a.nkv * DK) + a.eps) : 1.0f;
     const int partner = half / 8;                                    // lanes to the partner of a pair of halves: a power of two

@@ -111,3 +111,23 @@ def test_the_squares_of_a_head_are_added_in_their_order(nh, nkv, hd):
         s = s[..., :half] + s[..., half:]
     want = (x * (1.0 / torch.sqrt(s / hd + torch.tensor(eps, device=DEV)))) * gain
     assert torch.equal(out, want.to(torch.bfloat16).view(T, nh * hd))
+
+
+@pytest.mark.parametrize("nh,nkv,dk,wide_in", [(16, 4, 128, False), (32, 8, 64, True), (64, 16, 256, False)])
+def test_a_row_of_a_window_layer_does_not_depend_on_how_many_there_are(nh, nkv, dk, wide_in):
+    from llmengine_b200.kernels.ops import CudaOps
+    ops, g, ps, most = CudaOps(torch.device(DEV)), torch.Generator(device=DEV).manual_seed(nh), 16, 2500
+    rows = 3 * torch.randn(most, (nh + 2 * nkv) * dk, generator=g, device=DEV).to(torch.float32 if wide_in else torch.bfloat16)
+    qg, kg = [1 + 0.1 * torch.randn(n * dk, generator=g, device=DEV) for n in (nh, nkv)]
+    positions, outs = torch.arange(most, dtype=torch.int32, device=DEV), []
+    p = lambda t: c_void_p(t.data_ptr())
+    for T in (most, 700, 250, 100, 3):
+        kind = torch.float32 if wide_in else torch.bfloat16
+        cache, out = torch.zeros(-(-most // ps), 2 * ps * nkv * dk, device=DEV, dtype=kind), torch.zeros(most, nh * dk, device=DEV, dtype=kind)
+        args = _Post(p(rows), p(rows[:, nh * dk:]), p(rows[:, (nh + nkv) * dk:]), rows.stride(0), rows.stride(0), rows.stride(0), p(qg), p(kg), 1e-5, None, 0, 1.0,
+                     p(positions), p(out), p(cache), p(positions), T, nh, nkv, dk, dk, ps, None, None, None, 0, 0, int(wide_in), 0, 1)
+        ops.require("attention_window")
+        assert ops._lib("attention_window").llme_window_post(ctypes.byref(args), c_int(0 if wide_in else 1), c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        outs.append((out[:T].clone(), cache[:, :ps * nkv * dk].view(-1, nkv, ps, dk).transpose(1, 2).flatten(0, 1)[:T].clone()))
+    for q, k in outs[1:]:
+        assert torch.equal(q, outs[0][0][:len(q)]) and torch.equal(k, outs[0][1][:len(k)])
