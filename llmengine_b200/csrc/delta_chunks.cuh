@@ -371,7 +371,9 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) chunk_walk_kernel(const __gri
     auto before = [] { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); };
     auto publish = [] { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); };     // what the instructions read through the async proxy
 
-    if (warp < WALKERS) {
+    if (n_chunks <= 0) {
+        // ------------------------------------------------------------------ an empty portion: neither outputs nor a state to write
+    } else if (warp < WALKERS) {
         // ------------------------------------------------------------------ the walk: row `row` of S, token `tok` of the chunk, columns col .. col + MINE - 1
         const int row = tid & 127, tok = row & 63, col = (warp >> 2) * MINE;
         const bool keys = row < CHUNK;                             // lanes of K (and of N: r and u); the others of Q (and of B: the outputs)

@@ -59,6 +59,16 @@ def test_long_portions(lens, H, G, p, chunks):
         assert float((states[r].transpose(1, 2) - S).norm()) < TOL * float(S.norm()), r
 
 
+def test_empty_portions_beside_long_ones():
+    """They write nothing: outputs and states of the others are those of a step without them, and their own states stay."""
+    c = _case([0, 600, 0, 700, 0], 2, 1, 32, 11)
+    d = {**c, "lens": [600, 700], "state": c["state"][[0, 2, 4]]}        # (request r's state is slot len(lens) - r)
+    (y, states), (want, kept) = _go(c), _go(d)
+    assert torch.equal(y, want) and torch.equal(states[1], kept[0]) and torch.equal(states[3], kept[1])
+    for r in (0, 2, 4):
+        assert torch.equal(states[r], c["state"][5 - r])
+
+
 def test_values_that_are_not_finite_reach_no_token_before_them():
     lens, H, G, p = [400, 300], 2, 1, 64
     c = _case(lens, H, G, p, 7)
