@@ -30,8 +30,13 @@ constexpr int CHUNK = 64, N_ROWS = 128, P_COLS = 32;               // tokens; ro
 constexpr int COEF = 2 * CHUNK * CHUNK + 4 * CHUNK;                // floats per chunk and head: [N; B] as shared memory has it, then b, G and G(63, .) of every token
 
 __device__ __forceinline__ int request_of(const LlmeDeltaArgs& a, int place) { return a.rows ? a.rows[place] : place; }
-// Number of the first chunk of the portion at `place` among the rows: floor(first token / 64) + place (distinct for all chunks of a step).
-__device__ __forceinline__ int first_chunk(const LlmeDeltaArgs& a, int place) { return a.cu_q_lens[request_of(a, place)] / CHUNK + place; }
+// Number of the first chunk of the portion at `place` among the rows, distinct for all chunks of a step: floor(first token / 64) + place where
+// this form takes all portions (from = 0).  Where it takes those of LONG tokens and more (from = LONG), floor(first token / LONG) stands for the place,
+// which the shorter ones would push on: it grows by one at least from one of the others to the next.
+__device__ __forceinline__ int first_chunk(const LlmeDeltaArgs& a, int place, int from) {
+    const int t = a.cu_q_lens[request_of(a, place)];
+    return t / CHUNK + (from > 0 ? t / LONG : place);
+}
 
 // where element j of row i of [N; B] lies: two halves of 32 columns, 128-byte rows, their 16-byte pieces swizzled with the row
 __device__ __forceinline__ int nb_place(int i, int j) { return (j >> 5) * (2 * CHUNK * 32) + i * 32 + ((((j & 31) >> 2) ^ (i & 7)) << 2) + (j & 3); }
@@ -46,7 +51,7 @@ struct PrepareShared {
     float beta[2][CHUNK], keep[2][CHUNK];
 };
 
-__global__ void __launch_bounds__(PREPARE_THREADS, 2) chunk_prepare_kernel(LlmeDeltaArgs a) {
+__global__ void __launch_bounds__(PREPARE_THREADS, 2) chunk_prepare_kernel(LlmeDeltaArgs a, int from) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PrepareShared& sm = *reinterpret_cast<PrepareShared*>(smem_raw);
     pdl_launch_dependents();
@@ -55,10 +60,10 @@ __global__ void __launch_bounds__(PREPARE_THREADS, 2) chunk_prepare_kernel(LlmeD
     int place = 0, hi = a.n_rows;                                  // the last portion whose first chunk is not behind `id`
     while (hi - place > 1) {
         const int mid = (place + hi) >> 1;
-        if (first_chunk(a, mid) <= id) place = mid; else hi = mid;
+        if (first_chunk(a, mid, from) <= id) place = mid; else hi = mid;
     }
-    const int r = request_of(a, place), first = a.cu_q_lens[r], at = CHUNK * (id - first_chunk(a, place)), len = a.cu_q_lens[r + 1] - first;
-    if (at < 0 || at >= len) return;                               // a number no chunk has
+    const int r = request_of(a, place), first = a.cu_q_lens[r], at = CHUNK * (id - first_chunk(a, place, from)), len = a.cu_q_lens[r + 1] - first;
+    if (at < 0 || at >= len || len < from) return;                 // a number no chunk has, or a portion of the other form
     const int t0 = first + at, count = min(CHUNK, len - at);
     const int rep = a.heads / a.qk_groups, x = tid >> 7, t = tid & 127, j = tid & 63;
     const bool lower = !(tid & 64);
@@ -333,7 +338,7 @@ __device__ __forceinline__ void load_product(unsigned addr, float (&x)[MINE]) {
 
 constexpr size_t WALK_SMEM = 1024 + PIECES * KT_PLANE + PIECES * S_PLANE + 2 * PIECES * U_PLANE + KQ_RAW + NB_RAW + sizeof(WalkBarriers);
 
-__global__ void __launch_bounds__(WALK_THREADS, 1) chunk_walk_kernel(const __grid_constant__ CUtensorMap map_unit, LlmeDeltaArgs a) {
+__global__ void __launch_bounds__(WALK_THREADS, 1) chunk_walk_kernel(const __grid_constant__ CUtensorMap map_unit, LlmeDeltaArgs a, int from) {
     static_assert(DN_COL + P_COLS <= 512 && WALK_SMEM <= 232448, "sizes");
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -364,16 +369,18 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) chunk_walk_kernel(const __gri
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     pdl_wait();
     const int p0 = blockIdx.x * P_COLS, h = blockIdx.y, r = request_of(a, blockIdx.z), g = h / (a.heads / a.qk_groups);
-    const int first = a.cu_q_lens[r], len = a.cu_q_lens[r + 1] - first, n_chunks = (len + CHUNK - 1) / CHUNK, id0 = first_chunk(a, blockIdx.z);
+    const int first = a.cu_q_lens[r], len = a.cu_q_lens[r + 1] - first, n_chunks = (len + CHUNK - 1) / CHUNK, id0 = first_chunk(a, blockIdx.z, from);
+    if (len <= 0 || len < from) {                                  // an empty portion, or one of the other form: neither outputs nor a state to write
+        if (warp == WALK_ISSUER) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(bar->tmem_base), "r"(512u));
+        return;
+    }
     auto coef_of = [&](int c) { return a.coef + ((size_t)(id0 + c) * a.heads + h) * COEF; };
     const unsigned tmem = bar->tmem_base;
     auto after = [] { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); };
     auto before = [] { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); };
     auto publish = [] { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); };     // what the instructions read through the async proxy
 
-    if (n_chunks <= 0) {
-        // ------------------------------------------------------------------ an empty portion: neither outputs nor a state to write
-    } else if (warp < WALKERS) {
+    if (warp < WALKERS) {
         // ------------------------------------------------------------------ the walk: row `row` of S, token `tok` of the chunk, columns col .. col + MINE - 1
         const int row = tid & 127, tok = row & 63, col = (warp >> 2) * MINE;
         const bool keys = row < CHUNK;                             // lanes of K (and of N: r and u); the others of Q (and of B: the outputs)
@@ -638,24 +645,27 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) chunk_walk_kernel(const __gri
     }
 }
 
-// Whether these portions go 64 tokens at a time: what the forms above need of sizes and alignment, a workspace that holds the chunks, and
-// 256 tokens or more a portion on average.  Both forms, eight and 64 at a time (us): one portion of 200 tokens of 16 heads 40 and 44, of 300
-// 53 and 48, of 1,500 224 and 135; 20 of 48 81 and 103, four of 192 75 and 58; 32 heads, 16 of 100 248 and 236, four of 256 171 and 119.
-constexpr int LEAST_TOKENS = 256;
+// Whether portions can go 64 tokens at a time: what the forms above need of sizes and alignment, and a workspace that holds the chunks of
+// portions of LONG tokens or more.  Both forms, eight and 64 at a time (us): one portion of 200 tokens of 16 heads 40 and 44, of 300 53 and 48, of
+// 1,500 224 and 135; 20 of 48 81 and 103, four of 192 75 and 58; 32 heads, 16 of 100 248 and 236, four of 256 171 and 119.  LONG lies where they
+// meet for a portion by itself.  (Several shorter ones side by side would be faster here, but a portion is not to see what stands beside it.)
+int most_chunks(const LlmeDeltaArgs& a) { return a.tokens / CHUNK + a.tokens / LONG + 1; }
 bool takes(const LlmeDeltaArgs& a) {
     const uintptr_t all = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.out | (uintptr_t)a.unit | (uintptr_t)a.coef;
-    return a.n == N_ROWS && a.p % P_COLS == 0 && all % 16 == 0 && (a.ldq | a.ldk | a.ldv | a.ldo) % 4 == 0 &&
-           (long long)(a.tokens / CHUNK + a.n_rows + 1) * a.heads * COEF <= a.coef_floats && a.qk_groups <= 65535 && a.tokens / a.n_rows >= LEAST_TOKENS;
+    return a.n == N_ROWS && a.p % P_COLS == 0 && all % 16 == 0 && (a.ldq | a.ldk | a.ldv | a.ldo) % 4 == 0 && a.tokens >= LONG &&
+           (long long)most_chunks(a) * a.heads * COEF <= a.coef_floats && a.qk_groups <= 65535;
 }
 
-int launch(const LlmeDeltaArgs& a, cudaStream_t s) {
+// The portions of `from` = LONG tokens or more; 0: all, of which there are no more than a.tokens / LONG.
+int launch(const LlmeDeltaArgs& a, int from, cudaStream_t s) {
     static LlmeGrants prepare_grants, walk_grants;
     if (llme_grant_smem(prepare_grants, chunk_prepare_kernel, sizeof(PrepareShared)) != cudaSuccess || llme_grant_smem(walk_grants, chunk_walk_kernel, WALK_SMEM) != cudaSuccess)
         LLME_REFUSE("delta_rule: %zu bytes of shared memory are not available", WALK_SMEM);
-    llme_launch(chunk_prepare_kernel, dim3(a.tokens / CHUNK + a.n_rows + 1, a.qk_groups), dim3(PREPARE_THREADS), sizeof(PrepareShared), s, a);
     CUtensorMap unit;
     if (int rc = make_map(&unit, a.unit, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.tokens, 2LL * a.qk_groups * N_ROWS, 2LL * a.qk_groups * N_ROWS, CHUNK, 32)) return rc;
-    llme_launch(chunk_walk_kernel, dim3(a.p / P_COLS, a.heads, a.n_rows), dim3(WALK_THREADS), WALK_SMEM, s, unit, a);
+    llme_launch(chunk_prepare_kernel, dim3(from > 0 ? most_chunks(a) : a.tokens / CHUNK + a.n_rows + 1, a.qk_groups), dim3(PREPARE_THREADS), sizeof(PrepareShared), s, a, from);
+    llme_launch(chunk_walk_kernel, dim3(a.p / P_COLS, a.heads, a.n_rows), dim3(WALK_THREADS), WALK_SMEM, s, unit, a, from);
+    if (a.launches) *a.launches += 2;
     LLME_LAUNCH_STATUS();
 }
 

@@ -19,10 +19,11 @@
 // the inverse N of the unit lower triangular I + A, and B N, so that u = N r and o = G S0^T q + (B N) r: lane i of a column forms
 // u_i and o_i from the eight r's, and nothing is left to be solved in sequence.  No quotient of decays is ever formed, so a decay of
 // zero is harmless.  A block at a portion's end is filled up with tokens that change nothing (k = q = 0, b = 0, a = 1); how a
-// prompt is cut into steps changes the order of the sums and nothing else.  Long portions of heads with 128 rows go 64 tokens at a time
-// on the tensor cores instead (delta_chunks.cuh).
+// prompt is cut into steps changes the order of the sums and nothing else.  Portions of LONG tokens or more of heads with 128 rows go 64 tokens
+// at a time on the tensor cores instead (delta_chunks.cuh): a portion's own length decides, and what else is in the step changes no bit of it.
 #include <cuda.h>
 
+#include <climits>
 #include <type_traits>
 
 #include "common.cuh"
@@ -32,6 +33,7 @@ LLME_API const char* llme_last_error() { return llme_error_buffer(); }
 
 namespace {
 
+constexpr int LONG = 256;                        // tokens of a portion that goes 64 at a time
 constexpr int BLOCK = 8, ROW_NUMBERS = 20;       // tokens of a block; numbers that a token of a block and head needs: b, b G, G, G(7, .),
 constexpr int NUMBERS = BLOCK * ROW_NUMBERS;      // a row of N, a row of B N
 
@@ -206,7 +208,8 @@ __device__ __forceinline__ float sums_of_32(float (&v)[32], int lane) {
 // One warp per (block, query/key group).
 constexpr int PREPARE_WARPS = 4;
 
-__global__ void __launch_bounds__(32 * PREPARE_WARPS) delta_prepare_kernel(LlmeDeltaArgs a) {
+// (Here and in the walk: portions of `below` tokens or more are another form's.)
+__global__ void __launch_bounds__(32 * PREPARE_WARPS) delta_prepare_kernel(LlmeDeltaArgs a, int below) {
     // sums: [0, 36) k_j . q_i at i (i + 1) / 2 + j; [36, 64) k_j . k_i (j < i) at i (i - 1) / 2 + j; [64, 72) |q_i|^2; [72, 80) |k_i|^2
     __shared__ float sums_of[PREPARE_WARPS][96];
     pdl_launch_dependents();
@@ -219,7 +222,7 @@ __global__ void __launch_bounds__(32 * PREPARE_WARPS) delta_prepare_kernel(LlmeD
         if (first_block(a.cu_q_lens, mid) <= id) lo = mid; else hi = mid;
     }
     const int len = a.cu_q_lens[lo + 1] - a.cu_q_lens[lo], at = BLOCK * (id - first_block(a.cu_q_lens, lo));
-    if (at < 0 || at >= len || len < 2) return;                 // a number no block has, or a single token
+    if (at < 0 || at >= len || len < 2 || len >= below) return; // a number no block has, a single token, or another form's
     const int t0 = a.cu_q_lens[lo] + at, count = min(BLOCK, len - at), n = a.n, n4 = (n + 3) & ~3;
     float* sums = sums_of[warp];
     const float* qp = a.q + (size_t)t0 * a.ldq + (size_t)g * n;
@@ -321,7 +324,7 @@ struct DeltaTile {
 };
 
 template <int L, int M, int C, int W, int NS>
-__global__ void __launch_bounds__(32 * W) delta_tile_kernel(LlmeDeltaArgs a, int vec_state) {
+__global__ void __launch_bounds__(32 * W) delta_tile_kernel(LlmeDeltaArgs a, int vec_state, int below) {
     using Tile = DeltaTile<L, M, C, W, NS>;
     constexpr int ROW = Tile::ROW, COLS = Tile::COLS, P2 = 2 * M;         // packed pairs of rows a lane holds per column
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -330,6 +333,7 @@ __global__ void __launch_bounds__(32 * W) delta_tile_kernel(LlmeDeltaArgs a, int
     const int jb = blockIdx.x * COLS, mine = (warp * (32 / L) + lane / L) * C, col0 = jb + mine;
     const int h = blockIdx.y, r = a.rows ? a.rows[blockIdx.z] : (int)blockIdx.z, n = a.n, p = a.p, n4 = (n + 3) & ~3;
     const int first = a.cu_q_lens[r], last = a.cu_q_lens[r + 1], g = h / (a.heads / a.qk_groups);
+    if (last - first >= below) return;
     const int block0 = first_block(a.cu_q_lens, r);
     const float* uq = a.unit + (size_t)g * n4;
     const size_t ldu = (size_t)2 * a.qk_groups * n4, to_k = (size_t)a.qk_groups * n4;
@@ -479,7 +483,7 @@ __global__ void __launch_bounds__(32 * W) delta_tile_kernel(LlmeDeltaArgs a, int
 }
 
 template <int L, int M, int C, int W, int NS>
-int launch_tile(const LlmeDeltaArgs& a, int vec_state, cudaStream_t s) {
+int launch_tile(const LlmeDeltaArgs& a, int vec_state, int below, cudaStream_t s) {
     using Tile = DeltaTile<L, M, C, W, NS>;
     auto kernel = delta_tile_kernel<L, M, C, W, NS>;
     static LlmeGrants grants;
@@ -487,7 +491,7 @@ int launch_tile(const LlmeDeltaArgs& a, int vec_state, cudaStream_t s) {
         LLME_REFUSE("delta_rule: %zu bytes of shared memory are not available", sizeof(Tile));
     // An ordinary launch, which waits for the kernel before it: let in early, the blocks would crowd on the first SMs that have
     // room (there are about as many blocks as SMs), and the walk would take twice its time.
-    kernel<<<dim3((a.p + Tile::COLS - 1) / Tile::COLS, a.heads, a.n_rows), 32 * W, sizeof(Tile), s>>>(a, vec_state);
+    kernel<<<dim3((a.p + Tile::COLS - 1) / Tile::COLS, a.heads, a.n_rows), 32 * W, sizeof(Tile), s>>>(a, vec_state, below);
     LLME_LAUNCH_STATUS();
 }
 
@@ -521,25 +525,32 @@ LLME_API int llme_delta_step(const LlmeDeltaArgs* args, cudaStream_t stream) {
     LLME_LAUNCH_STATUS();
 }
 
-// The requests `rows`, each with two tokens or more, eight tokens at a time.
+// The requests `rows`, each with two tokens or more: eight tokens at a time, or 64 where a portion is long.  Where the portions are known to be
+// on one side of LONG, that side's form is launched alone and takes them all (also where a replayed step meets other lengths); else both are, one
+// after the other, and each passes over the other's portions.
 LLME_API int llme_delta_portions(const LlmeDeltaArgs* args, cudaStream_t stream) {
     const LlmeDeltaArgs& a = *args;
     if (a.n_rows <= 0) return 0;
     if (int rc = check(a)) return rc;
     if (!a.unit || !a.coef || ((uintptr_t)a.unit | (uintptr_t)a.coef) % 16) LLME_REFUSE("delta_rule: portions need their workspace");
-    if (chunks::takes(a)) return chunks::launch(a, stream);
+    const bool some_long = chunks::takes(a) && (a.longest <= 0 || a.longest >= LONG);
+    if (some_long && a.shortest >= LONG && a.n_rows <= a.tokens / LONG) return chunks::launch(a, 0, stream);
+    const int below = some_long ? LONG : INT_MAX;
     const dim3 blocks(a.tokens / BLOCK + a.requests + 1, (a.qk_groups + PREPARE_WARPS - 1) / PREPARE_WARPS);
-    llme_launch(delta_prepare_kernel, blocks, dim3(32 * PREPARE_WARPS), 0, stream, a);
+    llme_launch(delta_prepare_kernel, blocks, dim3(32 * PREPARE_WARPS), 0, stream, a, below);
     const int vs = rows_of_16(a.state, a.state_stride, a.n);
     // 16 columns a block either way: one a lane on four warps where there are few blocks (the walk's latency counts: 297 against
     // 350 us for 2,048 tokens of 16 heads of 128 x 128), two a lane on two warps where there are many (what is read from shared
     // memory counts: 410 against 465 us for 32 heads, 168 against 237 us for four requests of 512 tokens)
     const bool many = (long long)((a.p + 15) / 16) * a.heads * a.n_rows >= 200;
-    if (a.n <= 32) return many ? launch_tile<8, 1, 2, 2, 3>(a, vs, stream) : launch_tile<8, 1, 1, 4, 3>(a, vs, stream);
-    if (a.n <= 64) return many ? launch_tile<8, 2, 2, 2, 3>(a, vs, stream) : launch_tile<8, 2, 1, 4, 3>(a, vs, stream);
-    if (a.n <= 128) return many ? launch_tile<8, 4, 2, 2, 3>(a, vs, stream) : launch_tile<8, 4, 1, 4, 3>(a, vs, stream);
-    if (a.n <= 256) return launch_tile<16, 4, 1, 4, 3>(a, vs, stream);
-    return launch_tile<32, 4, 1, 4, 2>(a, vs, stream);
+    int rc;
+    if (a.n <= 32) rc = many ? launch_tile<8, 1, 2, 2, 3>(a, vs, below, stream) : launch_tile<8, 1, 1, 4, 3>(a, vs, below, stream);
+    else if (a.n <= 64) rc = many ? launch_tile<8, 2, 2, 2, 3>(a, vs, below, stream) : launch_tile<8, 2, 1, 4, 3>(a, vs, below, stream);
+    else if (a.n <= 128) rc = many ? launch_tile<8, 4, 2, 2, 3>(a, vs, below, stream) : launch_tile<8, 4, 1, 4, 3>(a, vs, below, stream);
+    else if (a.n <= 256) rc = launch_tile<16, 4, 1, 4, 3>(a, vs, below, stream);
+    else rc = launch_tile<32, 4, 1, 4, 2>(a, vs, below, stream);
+    if (a.launches) *a.launches += 2;
+    return rc || !some_long ? rc : chunks::launch(a, LONG, stream);
 }
 
 // 0, or where a bounded wait of the form that takes 64 tokens at a time gave up.

@@ -942,15 +942,16 @@ int op_delta_rule(LlmeExecutor& ex, const LlmeDeltaRuleOp& o, const LlmeStep& s,
     if (!step || !portions) return ex.fail("no delta_rule kernels are registered");
     LlmeDeltaArgs a = {o.q, o.k, o.v, o.ldq, o.ldk, o.ldv, o.write, o.forget, o.ld_gates, o.dt_bias, o.a_log, o.q_scale, o.unit_eps, o.state,
                        o.state_stride, o.out, o.ldo, s.cu_q_lens, s.state_slots, nullptr, s.num_requests, s.num_requests, s.num_tokens, o.heads,
-                       o.n, o.p, o.qk_groups, o.unit, o.coef, o.coef_floats};
+                       o.n, o.p, o.qk_groups, o.unit, o.coef, o.coef_floats, s.min_portion_len, s.max_portion_len, nullptr};
     if (ex.choice("delta_rule") == "tokens") return ex.launched(step(&a, st), "delta_step");      // every request, token after token
     if (s.num_portion > 0) {
         const long long n4 = (o.n + 3) / 4 * 4, blocks = s.num_tokens / 8 + s.num_requests + 1;
         if (s.num_tokens * 2 * o.qk_groups * n4 > o.unit_floats || blocks * o.heads * 160 > o.coef_floats)
             return ex.fail("delta_rule: the workspace is too small for %d tokens of %d requests", s.num_tokens, s.num_requests);
-        a.rows = s.portion_rows; a.n_rows = s.num_portion;
+        int kernels = 0;                                        // the blocks' numbers and the walk, of one form or of both
+        a.rows = s.portion_rows; a.n_rows = s.num_portion; a.launches = &kernels;
         if (int rc = ex.launched(portions(&a, st), "delta_portions")) return rc;
-        ++ex.launches;                                          // the blocks' numbers and the walk are two kernels
+        if (kernels > 1) ex.launches += kernels - 1;
     }
     if (s.num_decode > 0) {
         a.rows = s.decode_rows; a.n_rows = s.num_decode;

@@ -221,6 +221,8 @@ typedef struct LlmeDeltaArgs {
     int n_rows, requests, tokens, heads, n, p, qk_groups;
     float* unit; float* coef;                                /* workspace of portions: [T, 2 qk_groups n'], n' = n rounded up to fours; 160 values per block of 8 tokens and head */
     long long coef_floats;                                   /* what `coef` holds: with 8,448 values per chunk of 64 tokens and head, long portions go 64 tokens at a time */
+    int shortest, longest;                                   /* lengths of the shortest and longest of the portions `rows`, 0 where not known */
+    int* launches;                                           /* NULL, or a host counter that the kernels launched are added to */
 } LlmeDeltaArgs;
 
 /* The gates of a matrix memory with exponential gating (csrc/recurrent.cu), per request and head over the request's tokens:

@@ -1045,7 +1045,7 @@ private:
             int *tok = m, *pos = m + T_cap, *treq = m + 2 * T_cap, *slot = m + 3 * T_cap, *lrows = m + 4 * T_cap;
             int* cu = m + 5 * T_cap;
             int *ctx = cu + R_cap + 1, *slots = ctx + R_cap, *first = slots + R_cap, *dec = first + R_cap, *por = dec + R_cap;
-            int a = 0, nl = 0, nd = 0, np = 0, max_portion = 0, max_portion_ctx = 0, max_decode_ctx = 0;
+            int a = 0, nl = 0, nd = 0, np = 0, max_portion = 0, min_portion = 0, max_portion_ctx = 0, max_decode_ctx = 0;
             cu[0] = 0;
             for (int r = 0; r < R; ++r) {
                 const StepEntry& e = entries[r];
@@ -1068,6 +1068,7 @@ private:
                     max_decode_ctx = std::max(max_decode_ctx, s + 1);
                 } else {
                     por[np++] = r;
+                    min_portion = max_portion ? std::min(min_portion, n) : n;
                     max_portion = std::max(max_portion, n);
                     max_portion_ctx = std::max(max_portion_ctx, s + n);
                 }
@@ -1079,7 +1080,7 @@ private:
             }
             LlmeStep st = {};
             st.num_tokens = T; st.num_requests = R; st.num_logit_rows = NL; st.num_decode = nd; st.num_portion = np;
-            st.max_portion_len = max_portion; st.max_decode_ctx = max_decode_ctx; st.max_portion_ctx = max_portion_ctx;
+            st.min_portion_len = min_portion; st.max_portion_len = max_portion; st.max_decode_ctx = max_decode_ctx; st.max_portion_ctx = max_portion_ctx;
             int* d = meta_dev_;
             st.token_ids = d; st.positions = d + T_cap; st.token_request = d + 2 * T_cap; st.logit_rows = d + 4 * T_cap;
             int* dcu = d + 5 * T_cap;

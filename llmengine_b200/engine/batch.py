@@ -71,6 +71,10 @@ class StepBatch:
         return max((q for q in self.q_lens if q != 1), default=0)
 
     @property
+    def min_portion_len(self) -> int:
+        return min((q for q in self.q_lens if q != 1), default=0)
+
+    @property
     def max_portion_ctx(self) -> int:
         return max((s + q for s, q in zip(self.start_positions, self.q_lens) if q != 1), default=0)
 

@@ -63,6 +63,7 @@ typedef struct LlmeStep {
     LlmeStepGroup groups[LLME_MAX_GROUPS];
     int max_portion_ctx;       /* longest context among the requests with several tokens (0: not known); it decides between kernels of
                                   the same result, so a replay may meet others */
+    int min_portion_len;       /* shortest of the portions (0: not known, or one is empty); a replay may meet others */
 } LlmeStep;
 
 typedef int (*LlmeCallFn)(void* user, const LlmeStep* step, cudaStream_t stream);

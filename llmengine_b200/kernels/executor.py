@@ -46,7 +46,7 @@ class Step(Structure):
         ("token_ids", c_void_p), ("positions", c_void_p), ("token_request", c_void_p), ("cu_q_lens", c_void_p),
         ("ctx_lens", c_void_p), ("state_slots", c_void_p), ("first_portion", c_void_p), ("logit_rows", c_void_p),
         ("decode_rows", c_void_p), ("portion_rows", c_void_p), ("logits", c_void_p), ("blas", c_void_p),
-        ("num_groups", c_int), ("groups", StepGroup * MAX_GROUPS), ("max_portion_ctx", c_int),
+        ("num_groups", c_int), ("groups", StepGroup * MAX_GROUPS), ("max_portion_ctx", c_int), ("min_portion_len", c_int),
     ]
 
 

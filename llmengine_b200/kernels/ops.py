@@ -694,6 +694,7 @@ class CompiledPlan:
         s.num_decode, s.num_portion = batch.decode_rows.numel(), batch.portion_rows.numel()
         s.max_portion_len, s.max_decode_ctx = batch.max_portion_len, batch.max_decode_ctx
         s.max_portion_ctx = batch.max_portion_ctx if s.num_portion else 0
+        s.min_portion_len = batch.min_portion_len
         s.token_ids, s.positions, s.token_request = batch.token_ids.data_ptr(), batch.positions.data_ptr(), batch.token_request.data_ptr()
         s.cu_q_lens, s.ctx_lens, s.state_slots = batch.cu_q_lens.data_ptr(), batch.ctx_lens.data_ptr(), batch.state_slots.data_ptr()
         s.first_portion, s.logit_rows = batch.first_portion.data_ptr(), batch.logit_rows.data_ptr()

@@ -297,8 +297,8 @@ class Runtime:
         """What the delta rule over portions works from: the unit queries and keys of every token ([tokens, 2 * qk_heads * n'],
         n' = n rounded up to whole groups of four), and per block of eight tokens of a request and head the 160 numbers that
         its columns share (one buffer each for all layers; blocks are numbered floor(first token / 8) + place of the request in the
-        step + block of the request).  Portions of 256 tokens or more on average may instead go by chunks of 64 tokens where a head is
-        128, with 8,448 numbers per chunk and head; chunks are numbered alike, by place among the portions."""
+        step + block of the request).  Portions of 256 tokens or more go by chunks of 64 tokens where a head is 128, with 8,448 numbers per
+        chunk and head in the same memory, for tokens / 64 + tokens / 256 + 1 chunks (8,192 tokens of 32 heads: 174 MB)."""
         n4 = (n + 3) // 4 * 4
         blocks, chunks = self.max_tokens // 8 + self.max_requests + 1, self.max_tokens // 64 + self.max_tokens // 256 + 1
         need = max(blocks * heads * 160, chunks * heads * 8448 if n == 128 and self.max_tokens >= 256 else 0)

@@ -29,7 +29,7 @@ def _go(c, chunks=True):
     """Outputs [T, H, p] and states by request, from the kernels."""
     lens, H, G, p, T = c["lens"], c["H"], c["G"], c["p"], sum(c["lens"])
     x, gates, state = c["x"].to(DEV), c["gates"].to(DEV), c["state"].to(DEV)
-    floats = max((T // 8 + len(lens) + 1) * H * 160, (T // 64 + len(lens) + 1) * H * 8448 if chunks else 0)
+    floats = max((T // 8 + len(lens) + 1) * H * 160, (T // 64 + T // 256 + 1) * H * 8448 if chunks else 0)
     unit, coef, out = torch.full((T, 2 * G * N), float("nan"), device=DEV), torch.full((floats,), float("nan"), device=DEV), torch.zeros(T, H * p, device=DEV)
     slots = [len(lens) - r for r in range(len(lens))]
     _run(_ops(), lambda pl: pl.delta_rule(q=x[:, :G * N], k=x[:, G * N:2 * G * N], v=x[:, 2 * G * N:2 * G * N + H * p], write=gates[:, :H], forget=gates[:, H:],
@@ -57,6 +57,19 @@ def test_long_portions(lens, H, G, p, chunks):
                              beta, keep, c["state"][len(lens) - r].double().transpose(1, 2))
         assert float((y[s] - want).norm()) < TOL * float(want.norm()), r
         assert float((states[r].transpose(1, 2) - S).norm()) < TOL * float(S.norm()), r
+
+
+@pytest.mark.parametrize("lens", [[250] + [1] * 10 + [600], [700, 3, 2], [256, 255, 257, 2, 500], [40] * 9 + [300] + [7] * 30 + [900, 5, 256], [200, 210, 190, 255, 254]])
+def test_a_request_does_not_depend_on_its_neighbours(lens):
+    """Outputs and states of every request are those of a step that it has to itself, bit for bit."""
+    c = _case(lens, 4, 2, 64, sum(lens))
+    y, states = _go(c)
+    first = 0
+    for r, L in enumerate(lens):
+        s = slice(first, first + L)
+        first += L
+        own, kept = _go({**c, "lens": [L], "x": c["x"][s], "gates": c["gates"][s], "state": c["state"][[0, len(lens) - r]]})
+        assert torch.equal(y[s], own) and torch.equal(states[r], kept[0]), (r, L)
 
 
 def test_empty_portions_beside_long_ones():
