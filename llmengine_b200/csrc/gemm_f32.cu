@@ -427,7 +427,7 @@ int product(const float* A, const WT* W, float* C, int M, int N, int K, long lon
 
 }  // namespace
 
-// A [M,K] row stride lda; W [N,K] row stride ldw (float or bfloat16); C [M,N] row stride ldc.
+// A [M,K] row stride lda; W [N,K] row stride ldw (float or bfloat16); C [M,N] row stride ldc.  All of them may be what the kernel before writes.
 // `batch` products in one launch: member b reads A + b * sa and W + b * sw and writes C + b * sc.
 LLME_API int llme_gemm_nt_f32_batched(const float* A, const void* W, int w_dtype, float* C, int M, int N, int K, long long lda,
                                       long long ldw, long long ldc, int batch, long long sa, long long sw, long long sc,

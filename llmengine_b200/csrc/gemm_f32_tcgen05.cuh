@@ -57,6 +57,11 @@ template <bool SMALL> struct Shape {
     static_assert(STAGES * A_COLS + 2 * MAXN <= 512 && COLS % 8 == 0, "sizes");
 };
 
+// A request to bring a box into L2: it holds nothing back and may come ahead of what is written there.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+
 // What 32 bits give for one output: for outputs that the split does not reach.
 __device__ __noinline__ float plain_dot(const float* __restrict__ x, const float* __restrict__ w, int K) {
     float s = 0.0f;
@@ -216,8 +221,16 @@ gemm_nt_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, Args g) {
             __syncwarp();
         }
     } else {
-        // ------------------------------------------------------------------ raw weights (which no kernel before this one makes).  The whole warp waits and
-        // an elected lane asks: in one lane's branch a round of this took 1,350 cycles, and bounded everything.
+        // ------------------------------------------------------------------ raw weights.  The whole warp waits and an elected lane asks: in one lane's
+        // branch a round of this took 1,350 cycles, and bounded everything.
+        // (The kernel before may write what is taken for weights here: ahead of it goes only a request to have the first ones in L2.)
+        if (elect_one())
+            for (int c = 0; c < min(STAGES, chunks); ++c) {
+                tma_prefetch_2d(&map_w, (chunk0 + c) * CHUNK, n0);
+                tma_prefetch_2d(&map_w, (chunk0 + c) * CHUNK + 32, n0);
+            }
+        __syncwarp();
+        pdl_wait();
         int c = 0;
         for (; c < chunks; ++c) {
             const int b = c % STAGES;

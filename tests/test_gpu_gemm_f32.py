@@ -86,3 +86,20 @@ def test_no_number_where_32_bits_give_none_and_only_there():
         rest = torch.isfinite(exact) & ~large
         size = x.double().abs() @ w.double().abs().t()
         assert bool(((out.double() - exact).abs() <= (2 * 24 + 1024 + 8) * 2.0 ** -24 * size)[rest].all())
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 2048), (40, 2048, 1024), (3, 64, 512)])
+def test_weights_that_the_kernel_before_has_just_written(M, N, K):
+    """The norm in front lets its successor in early: what it writes is there all the same when it is taken for weights."""
+    from llmengine_b200.kernels.ops import CudaOps
+    ops, g = CudaOps(torch.device(DEV)), torch.Generator(device=DEV).manual_seed(N)
+    x, gain = torch.randn(M, K, generator=g, device=DEV), torch.ones(K, device=DEV)
+    w, out = torch.zeros(N, K, device=DEV), torch.empty(M, N, device=DEV)
+    for scale in (1.0, -1.0, 2.0, -3.0):
+        rows = torch.randn(N, K, generator=g, device=DEV)
+        want = scale * torch.nn.functional.rms_norm(rows.double(), (K,), eps=1e-6)
+        torch.cuda.synchronize()
+        ops.rmsnorm(rows, gain * scale, 1e-6, w)
+        ops.linear(x, w, out)
+        exact = x.double() @ want.t()
+        assert float((out.double() - exact).norm()) < 2e-6 * float(exact.norm()), scale
