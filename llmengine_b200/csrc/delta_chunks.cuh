@@ -315,7 +315,7 @@ __device__ __forceinline__ unsigned long long desc_rows128(const void* tile) {
 __device__ __forceinline__ void store_split(const float (&x)[MINE], unsigned char* tile, int row, int col, int plane) {
 #pragma unroll
     for (int i = 0; i < MINE / 8; ++i)
-        split8_to_smem(make_float4(x[8 * i], x[8 * i + 1], x[8 * i + 2], x[8 * i + 3]), make_float4(x[8 * i + 4], x[8 * i + 5], x[8 * i + 6], x[8 * i + 7]),
+        split8_to_smem<true>(make_float4(x[8 * i], x[8 * i + 1], x[8 * i + 2], x[8 * i + 3]), make_float4(x[8 * i + 4], x[8 * i + 5], x[8 * i + 6], x[8 * i + 7]),
                        tile + row * 64 + (((col / 8 + i) ^ ((row >> 1) & 3)) << 4), plane);
 }
 __device__ __forceinline__ void tmem_load16(unsigned addr, unsigned (&v)[16]) {
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) chunk_walk_kernel(const __gri
                 for (int i = 0; i < 4; ++i)
                     x[i] = real ? *reinterpret_cast<const float4*>(kq_raw + (t >> 6) * (KQ_RAW / 2) + (q >> 1) * (CHUNK * 128) + (t & 63) * 128 + ((((q & 1) * 4 + i) ^ (t & 7)) << 4))
                                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                split16_to_tmem(x, mine + KQ_COL + (unsigned)(q * 8), N_ROWS / 2);
+                split16_to_tmem<false>(x, mine + KQ_COL + (unsigned)(q * 8), N_ROWS / 2);
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             before();
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) chunk_walk_kernel(const __gri
                 float4 x[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(nb_raw + (q >> 1) * (NB_RAW / 2) + t * 128 + ((((q & 1) * 4 + i) ^ (t & 7)) << 4));
-                split16_to_tmem(x, mine + NB_COL + (unsigned)(q * 8), CHUNK / 2);
+                split16_to_tmem<false>(x, mine + NB_COL + (unsigned)(q * 8), CHUNK / 2);
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             before();
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) chunk_walk_kernel(const __gri
                     lo = *reinterpret_cast<const float4*>(src + (((2 * (q & 3)) ^ (tokn & 7)) << 4));
                     hi = *reinterpret_cast<const float4*>(src + (((2 * (q & 3) + 1) ^ (tokn & 7)) << 4));
                 }
-                split8_to_smem(lo, hi, kt + (q >> 3) * (CHUNK * 128) + tokn * 128 + (((q & 7) ^ (tokn & 7)) << 4), KT_PLANE);
+                split8_to_smem<false>(lo, hi, kt + (q >> 3) * (CHUNK * 128) + tokn * 128 + (((q & 7) ^ (tokn & 7)) << 4), KT_PLANE);
             }
             publish();
             __syncwarp();
@@ -577,8 +577,9 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) chunk_walk_kernel(const __gri
                 for (int i = 0; i < PAIRS; ++i)
 #pragma unroll
                     for (int k = part * steps / sums; k < (part + 1) * steps / sums; ++k)
-                        umma_from_tmem(tmem + d + (unsigned)(part * P_COLS), tmem + first_col + (unsigned)(PAIR_A[i] * step + k * 8),
-                                       b + (unsigned long long)(PAIR_B[i] * (plane >> 4) + k * 64), id_rows, i > 0 || k > part * steps / sums);
+                        umma_from_tmem(tmem + d + (unsigned)(part * P_COLS), tmem + first_col + (unsigned)(SecondUp::a(i) * step + k * 8),
+                                       b + (unsigned long long)(SecondUp::b(i) * (plane >> 4) + k * 64), id_rows, i > 0 || k > part * steps / sums,
+                                       k == part * steps / sums && SecondUp::steps_down(i));
         };
         for (int c = 0; c < n_chunks; ++c) {
             const unsigned now = (unsigned)c & 1;
@@ -603,8 +604,8 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) chunk_walk_kernel(const __gri
                 for (int i = 0; i < PAIRS; ++i)
 #pragma unroll
                     for (int k = 0; k < CHUNK / UMMA_K; ++k)
-                        umma_bf16(tmem + DN_COL, k_desc + (unsigned long long)(PAIR_A[i] * (KT_PLANE >> 4) + k * 128), r_desc + (unsigned long long)(PAIR_B[i] * (U_PLANE >> 4) + k * 64),
-                                  id_both, i > 0 || k > 0);
+                        umma_from_smem(tmem + DN_COL, k_desc + (unsigned long long)(SecondUp::a(i) * (KT_PLANE >> 4) + k * 128), r_desc + (unsigned long long)(SecondUp::b(i) * (U_PLANE >> 4) + k * 64),
+                                  id_both, i > 0 || k > 0, k == 0 && SecondUp::steps_down(i));
                 umma_commit(&bar->dn_done);
             }
             __syncwarp();

@@ -124,7 +124,7 @@ gemm_nt_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, Args g) {
             // (the instructions that read these columns are through: the copy waited for them)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int q = 0; q < 2; ++q) split16_to_tmem(f[q], mine + (unsigned)(b * A_COLS + q * 8), CHUNK / 2);
+            for (int q = 0; q < 2; ++q) split16_to_tmem<true>(f[q], mine + (unsigned)(b * A_COLS + q * 8), CHUNK / 2);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -159,7 +159,7 @@ gemm_nt_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, Args g) {
 #pragma unroll
             for (int j = 0; j < X_PIECES; ++j) {
                 const int row = row0 + X_ROWS * j;
-                if (row < nt) split8_to_smem(f[j][0], f[j][1], planes + b * PIECES * plane_bytes + row * 128 + ((q ^ (row & 7)) << 4), plane_bytes);
+                if (row < nt) split8_to_smem<true>(f[j][0], f[j][1], planes + b * PIECES * plane_bytes + row * 128 + ((q ^ (row & 7)) << 4), plane_bytes);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");           // the instructions read through the async proxy
             __syncwarp();
@@ -215,7 +215,7 @@ gemm_nt_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, Args g) {
                 for (int i = 0; i < PAIRS; ++i)
 #pragma unroll
                     for (int k = 0; k < CHUNK / UMMA_K; ++k)
-                        umma_from_tmem(d, a + (unsigned)(PAIR_A[i] * (CHUNK / 2) + k * 8), x + PAIR_B[i] * plane + 2 * k, id, i > 0 || k > 0);
+                        umma_from_tmem(d, a + (unsigned)(BothUp::a(i) * (CHUNK / 2) + k * 8), x + BothUp::b(i) * plane + 2 * k, id, i > 0 || k > 0, k == 0 && BothUp::steps_down(i));
                 umma_commit(&bar->done[b]);
             }
             __syncwarp();

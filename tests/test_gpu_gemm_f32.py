@@ -103,3 +103,19 @@ def test_weights_that_the_kernel_before_has_just_written(M, N, K):
         ops.linear(x, w, out)
         exact = x.double() @ want.t()
         assert float((out.double() - exact).norm()) < 2e-6 * float(exact.norm()), scale
+
+
+@pytest.mark.parametrize("x_power,w_power", [(-112, 0), (-118, 0), (-130, 0), (-140, 0), (0, -124), (0, -138), (-118, 100), (-128, 100), (120, -126), (-60, -60), (-63, -64), (-70, -72)])
+def test_operands_and_results_at_the_small_end(x_power, w_power):
+    """Operands keep all their bits as far as 32-bit numbers have them.  To the bound of ordinary products (above) comes what 32 bits cannot hold
+    of a small result: every addition may be off by 2^-149, the smallest number, 24 in a chunk and one for each chunk and segment."""
+    from llmengine_b200.kernels.ops import CudaOps
+    ops, g, N, K = CudaOps(torch.device(DEV)), torch.Generator(device=DEV).manual_seed(3), 256, 1024
+    x = (torch.randn(40, K, generator=g, device=DEV).double() * 2.0 ** x_power).float()
+    w = (torch.randn(N, K, generator=g, device=DEV).double() * 2.0 ** w_power).float()
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    bound = (2 * 24 + K / 64 + 5 + 1.5) * 2.0 ** -24 * size + (24 * (K / 64) + K / 64 + 5) * 2.0 ** -149
+    for M in (3, 40):
+        out = torch.empty(M, N, device=DEV)
+        ops.linear(x[:M], w, out)
+        assert bool(((out.double() - want[:M]).abs() <= bound[:M]).all()), M
