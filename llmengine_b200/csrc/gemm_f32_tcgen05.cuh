@@ -14,8 +14,8 @@
 // The segments of K (by K and N alone) are a cluster's blocks: each leaves its sums in shared memory and adds a share of the outputs over
 // the blocks in their order.  So an output's additions depend on K and N alone, and a row's bits on no other row.
 //
-// Infinities, NaN and values that overflow bfloat16 come out of the split as no number; an output that is none is formed again by multiply-adds
-// in the order of k, which gives what 32 bits give.
+// Infinities, NaN and values that overflow bfloat16 come out of the split as no number; an output that is none is formed again, from its rows
+// and in 64 bits, by the warp that stores it.
 //
 // Rows x outputs x values, us, with the multiply-adds before: 1 / 8 / 32 / 64 / 300 rows of 11008 x 2048 20.7 / 21.1 / 23.6 / 36 / 93 (19.1 / 28.7 / 70.7 /
 // 120 / 374), of 2048 x 5504 14.2 / 14.6 / 16.0 / 23 / 61 (17.4 / 24.1 / 47.9 / 76 / 201); 300 x 11008 x 2048 is 145 TFLOP/s (870 of bfloat16).  Error against 64 bits, 2-norm
@@ -62,12 +62,27 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, i
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
 
-// What 32 bits give for one output: for outputs that the split does not reach.
+// Outputs that the split does not reach, taken again by a whole warp from rows that begin on 16 bytes: whether a row holds a NaN (then nothing
+// else counts), and one output in 64 bits, whose rounding is infinite where the sum is too large and only there.
+__device__ __noinline__ bool row_has_nan(const float* __restrict__ x, int K) {
+    bool nan = false;
+#pragma unroll 4
+    for (int k = 4 * ((int)threadIdx.x & 31); k < K; k += 128) {
+        const float4 v = row_piece(x, k, K, true);
+        nan |= isnan(v.x) || isnan(v.y) || isnan(v.z) || isnan(v.w);
+    }
+    return __any_sync(0xffffffffu, nan);
+}
 __device__ __noinline__ float plain_dot(const float* __restrict__ x, const float* __restrict__ w, int K) {
-    float s = 0.0f;
-#pragma unroll 1
-    for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
-    return s;
+    double s = 0.0;
+#pragma unroll 4
+    for (int k = 4 * ((int)threadIdx.x & 31); k < K; k += 128) {
+        const float4 a = row_piece(x, k, K, true), b = row_piece(w, k, K, true);
+        s += ((double)a.x * b.x + (double)a.y * b.y) + ((double)a.z * b.z + (double)a.w * b.w);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return (float)s;
 }
 
 template <bool SMALL>
@@ -259,8 +274,8 @@ gemm_nt_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, Args g) {
     // a share of the outputs over all segments in their order
     const unsigned part = smem_u32(smem);
     for (int e = rank * THREADS + (int)threadIdx.x; e < nt * (BM / 4); e += g.segments * THREADS) {
-        const int m = m0 + e / (BM / 4), n = n0 + (e % (BM / 4)) * 4;
-        if (m >= g.M || n >= g.N) continue;
+        const int m = m0 + e / (BM / 4), n = n0 + (e % (BM / 4)) * 4;      // (a warp has one row)
+        if (m >= g.M) continue;
         float v[4];
         for (int from = 0; from < g.segments; ++from) {
             float4 f;
@@ -272,9 +287,24 @@ gemm_nt_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, Args g) {
             if (from == 0) { v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w; }
             else { v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w; }
         }
+        bool off = false;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (n + i < g.N && !isfinite(v[i])) v[i] = plain_dot(g.A + (size_t)m * g.lda, g.W + (size_t)(n + i) * g.ldw, g.K);
+        for (int i = 0; i < 4; ++i) off |= n + i < g.N && !isfinite(v[i]);
+        if (__any_sync(0xffffffffu, off)) {
+            const float* x = g.A + (size_t)m * g.lda;
+            const bool nan = row_has_nan(x, g.K);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const bool again = n + i < g.N && !isfinite(v[i]);
+                if (nan) { if (again) v[i] = __int_as_float(0x7fffffff); continue; }
+                for (unsigned left = __ballot_sync(0xffffffffu, again); left; left &= left - 1) {
+                    const int who = __ffs(left) - 1;
+                    const float d = plain_dot(x, g.W + (size_t)(__shfl_sync(0xffffffffu, n, who) + i) * g.ldw, g.K);
+                    if (lane == who) v[i] = d;
+                }
+            }
+        }
+        if (n >= g.N) continue;
         float* row = g.C + (size_t)m * g.ldc;
         if (g.vec_c && n + 4 <= g.N) *reinterpret_cast<float4*>(row + n) = make_float4(v[0], v[1], v[2], v[3]);
         else

@@ -119,3 +119,32 @@ def test_operands_and_results_at_the_small_end(x_power, w_power):
         out = torch.empty(M, N, device=DEV)
         ops.linear(x[:M], w, out)
         assert bool(((out.double() - want[:M]).abs() <= bound[:M]).all()), M
+
+
+@pytest.mark.parametrize("N,K", [(1000, 517), (11008, 2048)])
+def test_rows_that_are_no_numbers_do_not_hold_up_the_launch(N, K):
+    """A row of NaN, rows with one in their last place, an infinity: the outputs of 64 bits, at no more than forty times a launch of numbers (as
+    a serial sum a thread they took 260 times that)."""
+    from llmengine_b200.kernels.ops import CudaOps
+    ops, g = CudaOps(torch.device(DEV)), torch.Generator(device=DEV).manual_seed(N)
+    pad = -K % 4
+    clean, w = torch.randn(300, K + pad, generator=g, device=DEV), torch.randn(N, K + pad, generator=g, device=DEV)
+    every, some = clean.clone(), clean.clone()
+    every[:, :] = float("nan")
+    some[::3, K - 1], some[1, 5], some[2, 7] = float("nan"), float("inf"), 3.4e38
+    times = []
+    for x in (clean, every, some):
+        out = torch.empty(300, N, device=DEV)
+        took = []
+        for _ in range(4):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            ops.linear(x[:, :K], w[:, :K], out)
+            b.record()
+            torch.cuda.synchronize()
+            took.append(a.elapsed_time(b))
+        times.append(min(took[1:]))
+        exact = x[:, :K].double() @ w[:, :K].double().t()
+        want = exact.float()
+        assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out[want.isinf()], want[want.isinf()])
+    assert max(times[1:]) < 40 * times[0], times
