@@ -575,8 +575,10 @@ public:
             events.push_back({s.id, tok, s.phase == Phase::Finished, s.finish_reason});
         }
         // finished requests leave the batch and give back their pages and their slot at once
+        bool finished = false;
         for (size_t i = 0; i < active_.size();) {
             if (seqs_.at(active_[i]).phase == Phase::Finished) {
+                finished = true;
                 cache_->free_request(active_[i]);
                 finished_[active_[i]] = std::move(seqs_.at(active_[i]));
                 seqs_.erase(active_[i]);
@@ -585,7 +587,15 @@ public:
                 ++i;
             }
         }
+        if (finished) check_kernels();
         return events;
+    }
+
+    void check_kernels() override {
+        std::string gave_up;
+        for (auto& s : status_)                                      // (all of them: a flag left unread would speak up in a later call)
+            if (const int code = s.second()) gave_up += (gave_up.empty() ? "" : ", ") + s.first + " (code " + std::to_string(code) + ")";
+        if (!gave_up.empty()) throw Error("a wait inside a kernel gave up, the results are not valid: " + gave_up);
     }
 
     std::vector<int> generate(const std::vector<int>& prompt, int max_tokens, const SamplingParams& sp, int eos) override {
@@ -653,6 +663,11 @@ private:
         } else {
             reg("attention_plain", "attention_plain", "llme_attention_plain");
         }
+        // what says whether a bounded wait inside a library's kernels gave up
+        auto status = [&](const std::string& lib, const char* symbol) { status_.emplace_back(lib, (int (*)())libs_.symbol(lib, symbol)); };
+        if (dt_ == LLME_DT_F32) status("gemm_f32", "llme_gemm_f32_status");
+        else if (opt_.kernels == "fast") status("gemm_tcgen05", "llme_gemm_tc_status");
+        if (fast_attn && (cfg_.head_dim == 64 || cfg_.head_dim == 128)) status("attention_tc@HEAD_DIM=" + hd, "llme_attention_tc_status");
         sample_fn_ = (SampleFn)libs_.symbol("sampling", "llme_sample");
         penalty_fn_ = (PenaltyFn)libs_.symbol("sampling", "llme_repetition_penalty");
     }
@@ -1160,6 +1175,7 @@ private:
 
     EngineOptions opt_;
     KernelLibraries libs_;
+    std::vector<std::pair<std::string, int (*)()>> status_;
     ModelConfig cfg_;
     ExecutorApi x_ = {};
     LlmeExecutor* ex_ = nullptr;

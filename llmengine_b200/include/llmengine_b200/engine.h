@@ -103,7 +103,8 @@ public:
 
     /* Continuous batching: waiting -> prefilling -> decoding -> finished. */
     virtual long long submit(const Request& request) = 0;
-    virtual std::vector<TokenEvent> step() = 0;            /* admit, run one batch, sample, finish and free */
+    virtual std::vector<TokenEvent> step() = 0;            /* admit, run one batch, sample, finish and free; checks the kernels
+                                                              where a request finishes */
     virtual bool idle() const = 0;                         /* nothing active, nothing waiting */
     /* One prompt to its end (EOS or max_tokens): the generated tokens. */
     virtual std::vector<int> generate(const std::vector<int>& prompt_tokens, int max_tokens,
@@ -119,6 +120,9 @@ public:
     virtual int num_pages() const = 0;
     virtual long long kernel_launches() const = 0;
     virtual std::string architecture() const = 0;
+    /* Throws if a bounded wait inside a kernel has given up since the last call, so that results are not valid (waits for
+     * the device). */
+    virtual void check_kernels() = 0;
 };
 
 }  // namespace llmengine_b200
