@@ -723,8 +723,8 @@ __global__ void qkv_post_vec_kernel(QkvArgs a) {
 // token (its position's cosines and sines, its cache slot) is loaded once per warp instead of once per head; a lane holds 8 + 8 values
 // of a head (16-byte loads and stores), and all loads of its heads are on their way before the first is used.
 // Bound by latency, not by the 8 TB/s that its 50 MB would take at 2,048 tokens of 32 + 8 + 8 heads of 128: position and slot are looked
-// up in front of what depends on them, so a warp should have many bytes in flight.  That size takes 11.4 us, 17.5 with 8-byte pieces and twice
-// as many warps a token; 2,800 tokens of 16 + 4 + 4 heads 8.5 us and 12.5 (three heads a lane: 11.7 us, one: 14.3 us at the first size).
+// up in front of what depends on them, so a warp should have many bytes in flight.  That size takes 10.3 us, 15.0 with 8-byte pieces and twice
+// as many warps a token; 2,800 tokens of 16 + 4 + 4 heads 8.0 us and 10.7 (one and three heads a lane were 1.25 and 1.03 times slower).
 constexpr int QKV_WIDE_ITERS = 2;      // heads a lane takes part in
 constexpr int QKV_WIDE_WARPS = 8;      // = tokens per block
 
@@ -882,8 +882,11 @@ template <typename G>
 static bool launch_qkv_wide(const QkvArgs& a, cudaStream_t s) {
     const int heads = a.nh + 2 * a.nkv;
     if (a.hd != 32 && a.hd != 64 && a.hd != 128 && a.hd != 256) return false;
-    if (heads > 65535) return false;
-    if ((long long)a.tokens * heads * a.hd < 148LL * 16 * 512) return false;    // few tokens: a warp per (token, head)
+    const int pieces = 512 / a.hd, groups = (heads + pieces - 1) / pieces;      // runs of 512 values, of which a warp takes two
+    if (groups > 65535) return false;
+    // Few tokens: a warp per (token, head).  By whole runs, for small heads are costly there: 4,000 tokens of 3 + 3 + 3 heads of 32 take 12.4 us so,
+    // 3.9 here; 1,200 of 5 + 1 + 1 of 128 3.8 and 4.2.
+    if ((long long)a.tokens * groups < 148LL * 16) return false;
     if ((a.q_stride | a.k_stride | a.v_stride) & 3) return false;
     const uintptr_t ptrs = (uintptr_t)a.q_in | (uintptr_t)a.k_in | (uintptr_t)a.v_in | (uintptr_t)a.q_gain |
                            (uintptr_t)a.k_gain | (uintptr_t)a.cos_sin | (uintptr_t)a.q_out | (uintptr_t)a.k_out |

@@ -83,12 +83,20 @@ def test_rows_that_begin_on_eight_bytes(nh, nkv, hd):
     gain = 1 + 0.1 * torch.randn(hd, generator=g, device=DEV)
     table = torch.randn(T, hd, generator=g, device=DEV)
     positions = torch.arange(T, dtype=torch.int32, device=DEV)
+    x = whole.double().view(T, nh + 2 * nkv, hd)
+    u = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6) * gain.double()
+    a, b, c, s = u[..., :hd // 2], u[..., hd // 2:], table[:, None, :hd // 2].double(), table[:, None, hd // 2:].double()
+    want = torch.cat([a * c - b * s, a * s + b * c], -1)
+    # one rounding to bfloat16, and 32-bit sums and products before it
+    near = lambda got, to: bool(((got.double() - to).abs() <= BF16_STEP * to.abs() + 1e-5 * (1 + to.abs().amax(-1, keepdim=True))).all())
     outs = []
     for rows in (whole, odd[:, :n]):
         cache, out = torch.zeros(-(-T // page), 2, nkv, page, hd, device=DEV, dtype=torch.bfloat16), torch.zeros(T, nh * hd, device=DEV, dtype=torch.bfloat16)
         ops.qkv_post(q_in=rows[:, :nh * hd], k_in=rows[:, nh * hd:(nh + nkv) * hd], v_in=rows[:, (nh + nkv) * hd:], num_heads=nh, num_kv_heads=nkv, head_dim=hd, q_gain=gain,
                      k_gain=gain, eps=1e-6, cos_sin=table, positions=positions, q_out=out, cache=cache, slot_mapping=positions, page_size=page)
         outs.append((out, cache))
+        stored = cache.permute(0, 3, 1, 2, 4).reshape(-1, 2, nkv, hd)[:T]
+        assert near(out.view(T, nh, hd), want[:, :nh]) and near(stored[:, 0], want[:, nh:nh + nkv]) and torch.equal(stored[:, 1], whole.view(T, -1, hd)[:, nh + nkv:])
     assert float(outs[0][0].abs().max()) > 0 and torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
 
 
