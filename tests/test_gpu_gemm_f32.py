@@ -1,5 +1,5 @@
-"""The 32-bit product in each of its forms (weights streamed for up to 2, 4, 8, 16 and 32 rows, tiles of 128, 64 and 16 rows, whole and shared by a cluster) at sizes around their edges:
-against 64 bits, and bit for bit the same row whatever else is in the launch."""
+"""The 32-bit product in each of its forms (on the tensor cores; weights streamed for up to 2, 4, 8, 16 and 32 rows; tiles of 128, 64 and 16 rows, whole and shared by a cluster) at sizes
+around their edges: against 64 bits, and bit for bit the same row whatever else is in the launch."""
 import pytest
 import torch
 
@@ -9,9 +9,10 @@ DEV = "cuda:0"
 
 @pytest.mark.parametrize("N,K,w_dtype,pad", [
     (2048, 5504, torch.float32, 0), (1000, 1023, torch.float32, 0), (130, 2049, torch.bfloat16, 0), (64, 9001, torch.float32, 3), (11008, 2048, torch.float32, 0),
-    (300, 17, torch.bfloat16, 5), (4096, 16400, torch.bfloat16, 8), (50, 1030, torch.float32, 2), (4096, 16400, torch.float32, 4), (33, 6, torch.bfloat16, 2)])
+    (300, 17, torch.bfloat16, 5), (50, 4100, torch.float32, 4), (63, 2052, torch.float32, 0), (300, 3001, torch.float32, 2), (4096, 16400, torch.bfloat16, 8), (50, 1030, torch.float32, 2), (4096, 16400, torch.float32, 4), (33, 6, torch.bfloat16, 2)])
 def test_every_form(N, K, w_dtype, pad):
     from llmengine_b200.kernels.ops import CudaOps
+    # (float weights of 64 rows and 512 values or more whose rows begin on 16 bytes go to the tensor cores, all others to the multiply-adds)
     ops, g = CudaOps(torch.device(DEV)), torch.Generator(device=DEV).manual_seed(N + K)
     x = torch.randn(601, K + pad, generator=g, device=DEV)[:, :K]
     w = torch.randn(N, K + pad, generator=g, device=DEV).to(w_dtype)[:, :K]

@@ -61,6 +61,22 @@ def test_short_convolution_kernel(dtype, C, K):
     _check_short_convolution(dtype, C, K, [9, 1, 6], [4, 0, 5], 3)
 
 
+
+@pytest.mark.parametrize("channels", [128, 520])
+def test_convolution_weights_that_begin_on_four_bytes(channels):
+    """Four taps over many tokens: weights on 16 bytes are loaded four at a time, others one by one, to the same outputs."""
+    g = torch.Generator(device=DEV).manual_seed(channels)
+    x, b = torch.randn(300, channels, generator=g, device=DEV), torch.randn(channels, generator=g, device=DEV)
+    w, outs = torch.randn(channels, 4, generator=g, device=DEV), []
+    for shift in (0, 1):
+        place = torch.zeros(channels * 4 + 4, device=DEV)[shift:shift + channels * 4].view(channels, 4)
+        place.copy_(w)
+        state, out = torch.ones(2, 3, channels, device=DEV), torch.zeros(300, channels, device=DEV)
+        _run(_ops(), lambda p: p.short_conv(x=x, w=place, bias=b, state=state, out=out, act="silu"), _batch([200, 100], [1, 0]))
+        outs.append(out)
+    assert float(outs[0].abs().max()) > 0 and torch.equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("C,K", [(64, 4), (40, 3), (520, 2), (36, 5)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_short_convolution_over_long_portions(dtype, C, K):
