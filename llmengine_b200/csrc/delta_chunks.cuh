@@ -15,10 +15,11 @@
 //     Eight warps walk, eight split the next chunk's operands, one issues, one copies.
 // No quotient of decays is formed.  A chunk at a portion's end is filled up with tokens that change nothing (k = q = 0, b = 0, a = 1).
 // A value that is not finite would reach tokens before its own through the zeros of N and B: a block that meets one in u goes on token by token.
-// Bound by the chain of the four products of a chunk and the exchanges between them, some 6,700 cycles for 64 tokens, behind a preparation
-// that is bound by the 32-bit sums.  Two portions of 750 tokens, 16 heads of 128 x 128: 91 us, 157 us eight tokens at a time (the
-// preparation 41 us, of which 6 beside the walk); four of 375 with 32 heads 176 and 248, one of 2,048 with 32 heads 215 and 413.  Errors
-// against 64 bits, of the outputs 1.6e-7 (eight at a time 1.7e-7), of the state 1.2e-7 both.
+// Bound by the chain of the four products of a chunk and the exchanges between them, some 7,000 cycles for 64 tokens, behind a preparation
+// whose eleven warps an SM wait for shared memory and at barriers (its path is 32 % busy, the multiply-adds 23 %).  Two portions of 750 tokens, 16 heads of 128 x 128: 91 us, 157 us eight tokens at a
+// time (the preparation 41 us, of which 6 beside the walk); four of 375 with 32 heads 181 and 248, one of 2,048 with 32 heads 223 and 413.  Errors
+// against 64 bits, of the outputs 1.75e-7 (eight at a time 1.7e-7), of the state 1.2e-7 both.  (The tensor cores cut off what they add instead of
+// rounding it: that error has a sign, but goes no further than the 64 values of a sum, about 2^-24 of its largest part a step.)
 #pragma once
 
 namespace chunks {
@@ -647,9 +648,9 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) chunk_walk_kernel(const __gri
 }
 
 // Whether portions can go 64 tokens at a time: what the forms above need of sizes and alignment, and a workspace that holds the chunks of
-// portions of LONG tokens or more.  Both forms, eight and 64 at a time (us): one portion of 200 tokens of 16 heads 40 and 44, of 300 53 and 48, of
-// 1,500 224 and 135; 20 of 48 81 and 103, four of 192 75 and 58; 32 heads, 16 of 100 248 and 236, four of 256 171 and 119.  LONG lies where they
-// meet for a portion by itself.  (Several shorter ones side by side would be faster here, but a portion is not to see what stands beside it.)
+// portions of LONG tokens or more.  LONG lies where the forms meet for a portion by itself; eight and 64 at a time (us): 200 tokens of 16 heads 40 and
+// 44, 256 46 and 45, 300 52 and 48, 1,500 224 and 138; 32 heads 256 58 and 46, 300 68 and 51.  (Several shorter ones side by side would be faster
+// here, four of 192 58 against 68, but what stands beside a portion has no say.)
 int most_chunks(const LlmeDeltaArgs& a) { return a.tokens / CHUNK + a.tokens / LONG + 1; }
 bool takes(const LlmeDeltaArgs& a) {
     const uintptr_t all = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.out | (uintptr_t)a.unit | (uintptr_t)a.coef;

@@ -13,9 +13,9 @@
 //
 // 16 x 16 threads hold TM x TN outputs each, as packed pairs of neighbouring columns (fma.rn.f32x2: one instruction, each half
 // rounds as fmaf does); operands lie in shared memory k by k, two stages, the next one on its way through registers.
-// Bound by shared memory, whose path is 87 to 89 % busy while the multiply-adds fill 55 % of theirs: 300 x 11008 x 2048 takes 376 us and
-// 300 x 2048 x 5504 206 us (36 and 33 TFLOP/s of 74; 2,048 rows: 50 and 44); one block per 64 x 64 tile with 4 x 4 outputs a thread,
-// whatever the shape, took 675 and 617 us.
+// Bound by shared memory, whose path is 87 to 89 % busy while the multiply-adds fill 55 % of theirs.  All figures of this file are of float weights,
+// taken when these forms served them too: 300 x 11008 x 2048 took 376 us and 300 x 2048 x 5504 206 us (36 and 33 TFLOP/s of 74; 2,048 rows: 50 and
+// 44); one block per 64 x 64 tile with 4 x 4 outputs a thread, whatever the shape, took 675 and 617 us.
 // Up to 32 rows a third form streams the weights (further down).
 //
 // Reference counterparts: sgemm_nt_kernel (src/runtime/kernels/cuda_kernels.cu:282-294,
@@ -414,7 +414,7 @@ int product(const float* A, const WT* W, float* C, int M, int N, int K, long lon
         split::Args a = {A, (const float*)W, C, M, N, K, 0, 0, 0, g.vec_c, lda, ldw, ldc};
         return split::product(a, stream);
     }
-    // Few rows stream the weights: 32 rows take 73 and 50 us against 119 and 74 in tiles, 48 rows (two passes) 115 and 95 against 121
+    // Few rows stream the weights: 32 rows took 73 and 50 us against 119 and 74 in tiles, 48 rows (two passes) 115 and 95 against 121
     // and 78.  (Copies of four values need the alignment; the tiles take everything.)
     if (M <= FEW_ROWS && g.vec_a && g.vec_w) {
         if (M <= 2) return launch_few<WT, 2>(g, batch, stream);

@@ -17,13 +17,15 @@
 // Infinities, NaN and values that overflow bfloat16 come out of the split as no number; an output that is none is formed again, from its rows
 // and in 64 bits, by the warp that stores it.
 //
-// Rows x outputs x values, us, with the multiply-adds before: 1 / 8 / 32 / 64 / 300 rows of 11008 x 2048 20.7 / 21.1 / 23.6 / 36 / 93 (19.1 / 28.7 / 70.7 /
-// 120 / 374), of 2048 x 5504 14.2 / 14.6 / 16.0 / 23 / 61 (17.4 / 24.1 / 47.9 / 76 / 201); 300 x 11008 x 2048 is 145 TFLOP/s (870 of bfloat16).  Error against 64 bits, 2-norm
-// relative, 601 rows: 1.3e-7 and 1.2e-7 (5.7e-7 and 6.0e-7).
+// Rows x outputs x values, us, weights from memory, with the multiply-adds before: 1 / 8 / 32 / 64 / 300 rows of 11008 x 2048 21.9 / 22.0 / 25.0 / 36.9 / 95.5
+// (20.1 / 29 / 71 / 120 / 374), of 2048 x 5504 15.1 / 15.6 / 17.2 / 24.3 / 62.6 (17.8 / 24 / 48 / 76 / 201); 300 x 11008 x 2048 is 142 TFLOP/s (850 of bfloat16).  One
+// row of 11,008 outputs is the one slower case found: 86 blocks for 148 SMs.  1, 4 and 16 rows of 512 to 4,096 values on 64 to 4,096 outputs are 1.1 to
+// 3 times faster than the multiply-adds, so MIN_K and MIN_N need not be larger (64 x 512: 6.6 us, 7.2 to 11.8).  Error against 64 bits, 2-norm
+// relative, 601 rows: 1.3e-7 and 1.2e-7 (5.7e-7 and 6.0e-7); what the tensor cores cut off has a sign, but no sum there is longer than 64 values.
 // Few rows are bound by the eight warps that split the weights (about 1,000 cycles a chunk, 460 of them waits and barriers), many rows by the
 // instructions (1,340 cycles a chunk at 112 rows) and, where all SMs are at work, by what they bring from L2 (60 KB a chunk).  Tried: the sums
 // of x's and w's two tf32 parts (three products; error 3.7e-7, same times), pairs of SMs (1.2 times slower: an arrival at the partner's
-// barrier takes 425 cycles, one at the block's own 100), mma.sync with a few rows (the same bits, 26 us at 2048 x 2048 x 1: its chain of 24).
+// barrier takes 425 cycles, one at the block's own 100), mma.sync with a few rows (the same bits; one row of 2048 x 2048 26 us, 7.4 here: its chain of 24).
 // All waits are bounded; llme_gemm_f32_status() tells of one that gave up.
 #pragma once
 
